@@ -37,7 +37,7 @@
 namespace cg {
 
 constexpr uint32_t kLeafFlag = 0x80000000u;
-constexpr int kLeafCap = 96;        // buffered leaf pairs per traversal warp (a step adds up to 64)
+constexpr int kLeafCap = 96;        // buffered leaf pairs per warp of a traversal block (a step adds up to 64)
 constexpr int kChunk = 32;          // node pairs per donated task slot
 constexpr int kTraceBuckets = 512;  // utilisation trace: counters per time bucket
 
@@ -70,11 +70,12 @@ struct alignas(16) PackedQuery {
 };
 
 struct Counters {
-    unsigned int head;        // next task slot to claim (slots < n_queries are the root tasks)
-    unsigned int tail;        // one past the last reserved task slot
-    unsigned int done;        // finished tasks; all work is done when done == tail
+    unsigned int head;        // next donated slot to claim
+    unsigned int tail;        // one past the last reserved donated slot
+    unsigned int done;        // finished tasks; all work is done when done == n_queries + tail
     unsigned int error;       // ERR_* bits
-    unsigned int n_queries;   // queries of the launch (the next launch clears the slots it published)
+    unsigned int n_queries;   // queries of the launch
+    unsigned int root_next;   // next query whose root item no block has taken
     unsigned int narrow_lp;   // next leaf pair for the narrow phase
     unsigned long long n_pairs;
     unsigned long long n_leafs;
@@ -246,10 +247,9 @@ struct NarrowParams {
     uint32_t trace_ns;
 };
 
-// Work queue. A task is a chunk of up to kChunk node pairs: donated slot
-// s >= n_queries holds its chunk at pool[kChunk * (s - n_queries)], and
-// ready[s - n_queries] becomes count + 1 when it is published. Slot
-// s < n_queries is the root pair of query s.
+// Work queue. A task is the root item of a query, or a chunk of up to kChunk
+// items that a block gave away: donated slot s holds its chunk at
+// pool[kChunk * s], and ready[s] becomes count + 1 when it is published.
 struct TraverseParams {
     const PackedQuery* q;
     uint32_t n_queries;
@@ -257,7 +257,8 @@ struct TraverseParams {
     uint4* pool;          // node-pair entries (query, record a, record b, 0)
     unsigned int* ready;  // per donated slot
     uint32_t slot_cap;    // donated slots donors may reserve
-    uint32_t slot_alloc;  // allocated slots (slot_cap plus room for warps waiting past it)
+    uint32_t slot_alloc;  // allocated slots (slot_cap plus room for blocks waiting past it)
+    uint32_t root_batch;  // roots a block takes at a time
     Counters* ctr;
     uint4* leaf_list;     // (query, first triangle a, first triangle b, count_a | count_b << 16)
     uint32_t leaf_cap;
@@ -270,7 +271,15 @@ struct TraverseParams {
 };
 
 
-__host__ __device__ inline uint32_t warp_smem_words(uint32_t stack_cap) { return 3u * stack_cap + 4u * kLeafCap; }
+// Entries of the deque of a worker block of W (1, 2 or 4) warps. With
+// stack_cap >= 256 it is at least 64 W + 64, so that a step's pushes fit after
+// a forced donation.
+__host__ __device__ inline uint32_t deque_entries(uint32_t stack_cap, uint32_t W) {
+    return W >= 4u ? 2u * stack_cap : stack_cap;
+}
+__host__ __device__ inline uint32_t traverse_smem_words(uint32_t stack_cap, uint32_t W) {
+    return 3u * deque_entries(stack_cap, W) + 4u * kLeafCap * W;
+}
 constexpr uint32_t kNarrowWarpWords = 6u * 32u + 1u;  // a narrow block: 32 leaf pairs + prefix sums
 
 // Morph and skinning (cg_deform.cu); the arrays are those of cg_deform_view.

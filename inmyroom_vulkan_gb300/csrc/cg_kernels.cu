@@ -2,31 +2,36 @@
 // the persistent warp-cooperative OBB-tree traversal, and the persistent
 // triangle-pair (Moller) narrow phase.
 //
-// Traversal. Each warp owns a node-pair deque in shared memory and advances up
-// to 32 node pairs per step, one per lane: load both box records (four
-// 16-byte loads each) and the query's matrix in parallel, move B's box into
-// A's space, run the 15-axis SAT (three independent axes at a time), and apply
-// the reference's descent rule (OBBtree::IntersectOBBtreesRecursive,
-// src/Geometry/OBBtree.cpp:414-476): two inner nodes -> split the one with the
-// larger surface, ties to the first tree; one leaf -> split the other; two
-// leaves -> a candidate leaf pair. Surviving child pairs are pushed with
-// __ballot_sync/__popc compaction; candidate leaf pairs are buffered per warp
-// and appended to a global list in batches.
+// Traversal. A worker is a block of two or four warps that share a deque of
+// items in shared memory and advance it a step at a time: up to 32 items per
+// warp, an item being a split node whose two children are tested against the
+// other tree's box. A step loads the box records (four 16-byte loads each) and
+// the query's matrix, moves B's box into A's space, runs the 15-axis SAT (the
+// filter of cg_sat.cuh) and applies the reference's descent rule
+// (OBBtree::IntersectOBBtreesRecursive, src/Geometry/OBBtree.cpp:414-476): two
+// inner nodes -> split the one with the larger surface, ties to the first
+// tree; one leaf -> split the other; two leaves -> a candidate leaf pair.
+// Surviving child pairs are pushed with __ballot_sync/__popc compaction;
+// candidate leaf pairs are buffered per worker and appended to a global list
+// in batches.
 //
-// Load balance uses a global task queue. Tasks are chunks of up to 32 node
-// pairs; the root pairs of all queries are the first slots. A warp whose deque
-// runs dry claims the next slot and waits for it; a warp with fewer than 32
-// node pairs tops up with already reserved slots; a warp with surplus gives
-// half of the bottom (shallowest) part of its deque to waiting warps, with one
-// atomic per donation. Every wait is bounded by wait_ns (globaltimer), after
-// which the kernel records ERR_TIMEOUT and returns.
+// Load balance uses a global task queue. Tasks are the root items of the
+// queries, which the workers take first, and chunks of up to 32 items. A
+// worker whose deque runs dry claims the next chunk slot and waits for it; a
+// worker with surplus gives chunks from the bottom (shallowest) part of its
+// deque to waiting workers, with one atomic per donation. Every wait is
+// bounded by wait_ns (globaltimer), after which the kernel records
+// ERR_TIMEOUT and returns.
 //
 // Narrow phase. Each warp takes 32 leaf pairs of the list at a time and runs
 // their triangle pairs, one pair per lane.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "cg_device.cuh"
 #include "cg_internal.h"
+#include "cg_sat.cuh"
 
 namespace cg {
 
@@ -79,12 +84,13 @@ __device__ __forceinline__ unsigned long long* ht_of(Counters* c) {
 __device__ __forceinline__ uint32_t ht_head(unsigned long long v) { return uint32_t(v); }
 __device__ __forceinline__ uint32_t ht_tail(unsigned long long v) { return uint32_t(v >> 32); }
 
-// True once every reserved task has finished. `done` is read (acquire)
-// before the tail: done(t1) == tail(t2) with t1 < t2 implies no task was
-// running at t1 and none could be reserved afterwards.
-__device__ __forceinline__ bool all_done(Counters* c) {
-    const unsigned d = ld_acquire(&c->done);
-    return d == ht_tail(ld_relaxed64(ht_of(c)));
+// True once every task (the queries' roots and the donated chunks) has
+// finished. `done` is read (acquire) before the tail: done(t1) == n_queries +
+// tail(t2) with t1 < t2 implies no task was running at t1 and none could be
+// reserved afterwards.
+__device__ __forceinline__ bool all_done(const TraverseParams& P) {
+    const unsigned d = ld_acquire(&P.ctr->done);
+    return d == P.n_queries + ht_tail(ld_relaxed64(ht_of(P.ctr)));
 }
 
 struct Rec {
@@ -125,113 +131,59 @@ __device__ __forceinline__ void load_tri(const float4* tris, uint32_t i, float3&
     p2 = make_float3(c.x, c.y, c.z);
 }
 
-// Round g of the 15 axes of cg::sat (same axes, same order, same arithmetic):
-// g = 0 a's faces, 1 b's faces, 2..4 a_u|a_v|a_w x b_u, b_v, b_w.
-__device__ __forceinline__ bool sat_round(const Box& a, const Box& b, int g) {
-    float3 x0, y0, x1, y1, x2, y2;
-    if (g < 2) {
-        const float3 u = g ? b.u : a.u;
-        const float3 v = g ? b.v : a.v;
-        const float3 w = g ? b.w : a.w;
-        x0 = v;
-        y0 = w;
-        x1 = u;
-        y1 = w;
-        x2 = u;
-        y2 = v;
-    } else {
-        const float3 e = g == 2 ? a.u : (g == 3 ? a.v : a.w);
-        x0 = e;
-        y0 = b.u;
-        x1 = e;
-        y1 = b.v;
-        x2 = e;
-        y2 = b.w;
-    }
-    const bool ok0 = overlap_on(a, b, cross3(x0, y0));
-    const bool ok1 = overlap_on(a, b, cross3(x1, y1));
-    const bool ok2 = overlap_on(a, b, cross3(x2, y2));
-    return ok0 & ok1 & ok2;
+// Whether boxes a and b overlap on every axis of `open` (bits as sat_axis
+// numbers them): the filter's undecided axes, 1 in 3,000 box pairs.
+__device__ __noinline__ bool overlap_on_axes(const Box& a, const Box& b, unsigned open) {
+    do {
+        const uint32_t k = uint32_t(__ffs(int(open))) - 1u;
+        if (!sat_axis(a, b, k)) return false;
+        open &= open - 1u;
+    } while (open);
+    return true;
 }
+__device__ __noinline__ float surface_of(const Box& b) { return surface(b); }
 
-// Two box-pair SATs side by side, round by round, for instruction-level
-// parallelism; each verdict is the conjunction of its 15 axes, identical to
-// cg::sat.
-__device__ __forceinline__ void sat_two(const Box& a0, const Box& b0, const Box& a1, const Box& b1, bool& ok0,
-                                        bool& ok1) {
-    bool al0 = ok0, al1 = ok1;
-#pragma unroll 1
-    for (int g = 0; g < 5 && (al0 | al1); ++g) {
-        const bool r0 = sat_round(a0, b0, g);
-        const bool r1 = sat_round(a1, b1, g);
-        al0 = al0 & r0;
-        al1 = al1 & r1;
-    }
-    ok0 = al0;
-    ok1 = al1;
-}
-
-// Axis k (0..14) of the SAT in the reference's order: a's face normals
-// (v x w, u x w, u x v), b's, then a_i x b_j; true when the boxes overlap on
-// it. The SAT verdict is the conjunction over k, whatever lanes compute it.
-__device__ __forceinline__ bool sat_axis(const Box& a, const Box& b, uint32_t k) {
-    float3 x, y;
-    if (k < 6u) {
-        const bool onA = k < 3u;
-        const uint32_t f = onA ? k : k - 3u;
-        const float3 u = onA ? a.u : b.u, v = onA ? a.v : b.v, w = onA ? a.w : b.w;
-        x = f == 0u ? v : u;
-        y = f == 2u ? v : w;
-    } else {
-        const uint32_t i = (k - 6u) / 3u, j = (k - 6u) % 3u;
-        x = i == 0u ? a.u : (i == 1u ? a.v : a.w);
-        y = j == 0u ? b.u : (j == 1u ? b.v : b.w);
-    }
-    return overlap_on(a, b, cross3(x, y));
-}
+// What a child pair gives: an item, a candidate leaf pair or (kNone) nothing,
+// with its three words.
+enum : int { kNone = 0, kItem = 1, kLeaf = 2 };
+struct Out {
+    int what;
+    uint32_t q, s, o;
+};
 
 // The reference descent rule (OBBtree.cpp:414-476) for a child pair whose
 // boxes overlap: split the inner node with the larger box surface (the first
 // tree's on ties), else the inner one, or report a leaf pair. C is the child
 // record (record rc) of the split node, O the other box (record io), bx the
-// child pair's box of the second tree as transformed for the SAT.
-__device__ __forceinline__ void descend(const TraverseParams& P, bool sideB, const Rec& O, const Rec& C, uint32_t rc,
-                                        uint32_t io, uint32_t qi, const Box& bx, bool& item, bool& leaf,
-                                        uint32_t& out_q, uint32_t& out_s, uint32_t& out_o) {
+// child pair's box of the second tree as transformed for the SAT; `surf` is
+// within `surf_err` of its surface (the surface itself is computed only where
+// that does not settle the comparison).
+__device__ __forceinline__ Out descend(const TraverseParams& P, bool ok, bool sideB, const Rec& O, const Rec& C,
+                                       uint32_t rc, uint32_t io, uint32_t qi, const Box& bx, float surf,
+                                       float surf_err) {
     const uint32_t a_ref = sideB ? O.ref : C.ref;
     const uint32_t a_meta = sideB ? O.meta : C.meta;
     const float a_surf = sideB ? O.surf : C.surf;
     const uint32_t b_ref = sideB ? C.ref : O.ref;
     const uint32_t b_meta = sideB ? C.meta : O.meta;
-    const uint32_t ra = sideB ? io : rc;
-    const uint32_t rb = sideB ? rc : io;
     const bool la = (a_meta & kLeafFlag) != 0;
     const bool lb = (b_meta & kLeafFlag) != 0;
-    int act;  // 1: split A, 2: split B, 3: leaf pair
-    if (!la && !lb)
-        act = (a_surf >= surface(bx)) ? 1 : 2;
-    else if (la && !lb)
-        act = 2;
-    else if (!la && lb)
-        act = 1;
-    else
-        act = 3;
-    if (act == 3) {
-        // leaf pair: first triangles of both leaves, counts packed
-        leaf = true;
-        out_s = a_ref;
-        out_o = b_ref;
-        out_q = (a_meta & 0xffffu) | ((b_meta & 0xffffu) << 16);
-    } else {
-        item = true;
-        const uint32_t split = act == 1 ? a_ref : b_ref;
-        out_q = act == 1 ? qi : (qi | kItemSideB);
-        out_s = split;
-        out_o = act == 1 ? rb : ra;
-        // the split node's two child records share one 128-byte line: fetch
-        // it into L1 for the step that tests them
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.recs + 4ull * split));
-    }
+    const float diff = a_surf - surf;
+    bool larger = diff > 0.0f;
+    if (ok && !la && !lb && !(fabsf(diff) > surf_err)) larger = a_surf >= surface_of(bx);
+    const bool split_a = !la && (lb || larger);
+    const bool both = la && lb;
+    Out r;
+    r.what = !ok ? kNone : (both ? kLeaf : kItem);
+    // a leaf pair: first triangles of both leaves, counts packed; an item: the
+    // split node's first child, the other record, the query and side
+    r.q = both ? (a_meta & 0xffffu) | (b_meta << 16) : (split_a ? qi : (qi | kItemSideB));
+    r.s = (both || split_a) ? a_ref : b_ref;
+    r.o = both ? b_ref : (split_a == sideB ? rc : io);
+    // the split node's two child records share one 128-byte line: fetch it
+    // into L1 for the step that tests them
+    if (r.what == kItem) asm volatile("prefetch.global.L1 [%0];" ::"l"(P.recs + 4ull * r.s));
+    return r;
 }
 
 struct Deque {
@@ -241,65 +193,23 @@ struct Deque {
     uint32_t mask;
 };
 
-// Lane 0: one look at slot `slot`: 1 with r = its chunk size + 1 (2 for a
-// root slot) when it can be read, 0 with r = 0
-// when all work finished, an error was raised or the wait limit (counted
-// from t0) passed, -1 when it is not ready yet.
+// One look at donated slot `slot`: 1 with r = its chunk size + 1 when it can
+// be read, 0 with r = 0 when all work finished, an error was raised or the
+// wait limit (counted from t0) passed, -1 when it is not ready yet.
 __device__ int poll_ready(const TraverseParams& P, uint32_t slot, unsigned long long t0, unsigned& r) {
     r = 0;
-    if (slot < P.n_queries) {
-        r = 2u;
-        return 1;
-    }
-    const uint32_t idx = slot - P.n_queries;
-    if (idx < P.slot_alloc) {
-        r = ld_acquire(P.ready + idx);
+    if (slot < P.slot_alloc) {
+        r = ld_acquire(P.ready + slot);
         if (r) return 1;
     }
     // past every slot a donor could publish, only the end of the work or an
-    // error releases the warp
-    if (all_done(P.ctr) || ld_relaxed(&P.ctr->error) != 0) return 0;
+    // error releases the block
+    if (all_done(P) || ld_relaxed(&P.ctr->error) != 0) return 0;
     if (gtimer() - t0 > P.wait_ns) {
         atomicOr(&P.ctr->error, ERR_TIMEOUT);
         return 0;
     }
     return -1;
-}
-
-// Copies the chunk of slot `slot` into the deque at `top` (all lanes); `r` is
-// poll_ready's value. Returns the number of node pairs added.
-__device__ uint32_t take_chunk(const TraverseParams& P, uint32_t slot, unsigned r, const Deque& D, uint32_t top,
-                               int lane) {
-    // Lane 0 observed the slot's release; the barrier orders the other lanes'
-    // pool reads after that acquire.
-    __syncwarp();
-    uint32_t cnt = 0;
-    if (slot >= P.n_queries) {
-        cnt = r - 1u;
-        if (uint32_t(lane) < cnt) {
-            const uint4 e = ld_relaxed4(P.pool + size_t(kChunk) * (slot - P.n_queries) + lane);
-            const uint32_t pos = (top + lane) & D.mask;
-            D.q[pos] = e.x;
-            D.a[pos] = e.y;
-            D.b[pos] = e.z;
-        }
-    } else {
-        // the first item of query `slot`, made by the pack kernel
-        uint32_t iq = kNoItem;
-        if (lane == 0) {
-            const PackedQuery* Q = P.q + slot;
-            iq = __ldg(&Q->item_q);
-            if (iq != kNoItem) {
-                const uint32_t pos = top & D.mask;
-                D.q[pos] = iq;
-                D.a[pos] = __ldg(&Q->item_split);
-                D.b[pos] = __ldg(&Q->item_other);
-            }
-        }
-        cnt = __shfl_sync(kFull, iq != kNoItem ? 1u : 0u, 0);
-    }
-    __syncwarp();
-    return cnt;
 }
 
 __device__ __forceinline__ void trace_add(unsigned int* trace, uint32_t trace_ns, unsigned long long t_base, int field,
@@ -457,91 +367,154 @@ __device__ __forceinline__ void narrow_block(const NarrowParams& P, uint32_t* st
     __syncwarp();
 }
 
-// Appends the warp's buffered leaf pairs to the list.
-__device__ __forceinline__ void flush_leafs(const TraverseParams& P, const uint32_t* lq, const uint32_t* loa,
-                                            const uint32_t* lob, const uint32_t* lcn, uint32_t nl, int lane) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&P.ctr->n_leafs, (unsigned long long)nl);
-    base = __shfl_sync(kFull, base, 0);
-    for (uint32_t e = lane; e < nl; e += 32)
+// The words a block's threads share beside its deque and leaf buffer.
+struct TraverseShared {
+    unsigned push[2];             // this step's pushes so far: items | leaf pairs << 16 (by step parity)
+    unsigned long long qs[2];     // the queue's head and tail as read in the step (by step parity)
+    unsigned long long leaf_base; // where a flush goes in the list
+    uint32_t claim;               // first root or donated slot taken, roots or chunk size taken; 0: the end
+    uint32_t claim_n;
+    uint32_t claim_root;
+    int mode;                     // the donation: slots reserved (1), none (0), queue full (-1)
+    uint32_t slot;
+};
+
+// Appends the block's buffered leaf pairs to the list (all threads).
+__device__ __forceinline__ void flush_leafs(const TraverseParams& P, TraverseShared& sh, const uint32_t* lq,
+                                            const uint32_t* loa, const uint32_t* lob, const uint32_t* lcn,
+                                            uint32_t nl) {
+    if (threadIdx.x == 0) sh.leaf_base = atomicAdd(&P.ctr->n_leafs, (unsigned long long)nl);
+    __syncthreads();
+    const unsigned long long base = sh.leaf_base;
+    for (uint32_t e = threadIdx.x; e < nl; e += blockDim.x)
         if (base + e < P.leaf_cap) P.leaf_list[base + e] = make_uint4(lq[e], loa[e], lob[e], lcn[e]);
-    __syncwarp();
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(256, 2) traverse_kernel(const TraverseParams P) {
+constexpr uint32_t kWorkerMax = 4;  // warps of the widest worker block
+
+// A block of W warps is one worker: its warps share a deque of items in
+// shared memory and advance it together, one step (two barriers) at a time.
+__global__ void __launch_bounds__(kWorkerMax * 32, 2) traverse_kernel(const TraverseParams P) {
     extern __shared__ uint32_t smem[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const uint32_t S = P.stack_cap;
+    __shared__ TraverseShared sh;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t NT = blockDim.x, W = NT >> 5;
+    const uint32_t S = deque_entries(P.stack_cap, W);
     Deque D;
-    D.q = smem + size_t(warp) * warp_smem_words(S);
+    D.q = smem;
     D.a = D.q + S;
     D.b = D.a + S;
     D.mask = S - 1u;
     uint32_t* lq = D.b + S;
-    uint32_t* loa = lq + kLeafCap;
-    uint32_t* lob = loa + kLeafCap;
-    uint32_t* lcn = lob + kLeafCap;
+    uint32_t* loa = lq + kLeafCap * W;
+    uint32_t* lob = loa + kLeafCap * W;
+    uint32_t* lcn = lob + kLeafCap * W;
     unsigned long long* ht = ht_of(P.ctr);
 
-    uint32_t top = 0, bot = 0, nl = 0, held_tasks = 0;
+    // the block's state, the same in every thread
+    uint32_t top = 0, bot = 0, nl = 0, held_tasks = 0, par = 0;
+    bool roots_left = true;
     unsigned long long st_nodes = 0, st_don = 0, st_steps = 0;
     unsigned long long t_base = 0;
-    if (P.trace && lane == 0) t_base = trace_base(P.ctr);
+    if (P.trace && tid == 0) t_base = trace_base(P.ctr);
+    if (tid < 2u) sh.push[tid] = 0u;
 
     for (;;) {
         if (top == bot) {
-            // Out of work: claim the next slot and wait for it (the whole
-            // warp polls; lane 0 looks and sleeps between looks).
-            uint32_t slot = 0;
-            if (lane == 0) slot = ht_head(atomicAdd(ht, 1ull));
-            slot = __shfl_sync(kFull, slot, 0);
-            unsigned r = 0;
-            unsigned long long t0 = 0;
-            unsigned ns = 32;
-            for (;;) {
-                int st = 0;
-                if (lane == 0) {
-                    if (!t0) t0 = gtimer();
-                    st = poll_ready(P, slot, t0, r);
+            // Out of work: take the next roots, or claim the next donated slot
+            // and wait for it (thread 0 looks and sleeps between looks, the
+            // others wait at the barrier).
+            if (tid == 0) {
+                uint32_t n = 0, at = 0, root = 0;
+                if (roots_left) {
+                    at = atomicAdd(&P.ctr->root_next, P.root_batch);
+                    if (at < P.n_queries) {
+                        n = min(P.root_batch, P.n_queries - at);
+                        root = 1u;
+                    }
                 }
-                st = __shfl_sync(kFull, st, 0);
-                if (st >= 0) break;
-                if (lane == 0) {
-                    __nanosleep(ns);
-                    if (ns < kPollSleepMaxNs) ns <<= 1;
+                if (!root) {
+                    at = ht_head(atomicAdd(ht, 1ull));
+                    unsigned r = 0;
+                    const unsigned long long t0 = gtimer();
+                    unsigned ns = 32;
+                    while (poll_ready(P, at, t0, r) < 0) {
+                        __nanosleep(ns);
+                        if (ns < kPollSleepMaxNs) ns <<= 1;
+                    }
+                    n = r ? r - 1u : 0u;
                 }
-                __syncwarp();
+                sh.claim = at;
+                sh.claim_n = n;
+                sh.claim_root = root;
             }
-            r = __shfl_sync(kFull, r, 0);
-            if (!r) break;
-            top += take_chunk(P, slot, r, D, top, lane);
-            held_tasks = 1;
+            __syncthreads();
+            const uint32_t at = sh.claim, cn = sh.claim_n;
+            if (cn == 0u) break;
+            roots_left = sh.claim_root != 0u;
+            held_tasks = roots_left ? cn : 1u;
+            if (roots_left) {
+                // the first items of queries [at, at + cn), made by the pack kernel
+                for (uint32_t k = tid; k < cn; k += NT) {
+                    const PackedQuery* Q = P.q + at + k;
+                    const uint32_t iq = __ldg(&Q->item_q);
+                    if (iq != kNoItem) {
+                        const uint32_t pos = atomicAdd(&sh.push[par], 1u) & D.mask;  // the deque is empty: top is 0
+                        D.q[pos] = iq;
+                        D.a[pos] = __ldg(&Q->item_split);
+                        D.b[pos] = __ldg(&Q->item_other);
+                    }
+                }
+                __syncthreads();
+                bot = 0;
+                top = sh.push[par];
+                __syncthreads();
+                if (tid == 0) sh.push[par] = 0u;
+                if (top == 0u) {
+                    if (tid == 0) atomicAdd(&P.ctr->done, held_tasks);
+                    __syncthreads();
+                    continue;
+                }
+            } else {
+                // thread 0 observed the slot's release; the barrier orders the
+                // other threads' pool reads after that acquire
+                if (tid < cn) {
+                    const uint4 e = ld_relaxed4(P.pool + size_t(kChunk) * at + tid);
+                    D.q[tid] = e.x;
+                    D.a[tid] = e.y;
+                    D.b[tid] = e.z;
+                }
+                bot = 0;
+                top = cn;
+            }
+            __syncthreads();
         }
 
         // Queue state, read early so its latency overlaps the step's loads.
         unsigned long long qs = 0;
-        if (lane == 0) qs = ld_relaxed64(ht);
+        if (tid == 0) qs = ld_relaxed64(ht);
 
-        // ---- one step over up to 32 items from the top of the deque. An item
+        // ---- one step over up to 32 W items from the top of the deque. An item
         // tests both children of a split node against the other box: the
         // other record is loaded (and, for the second tree, transformed) once,
         // the two child records come from one 128-byte line. With more than
-        // 16 items a lane runs an item's two SATs side by side; with fewer,
-        // 2 L lanes share an item, L per child (L = 1, 2, 4, 8, 16 for 9-16,
-        // 5-8, 3-4, 2 and 1 items), each taking every L-th of the child's 15
-        // axes, so that a step with few items (the ramp and the tail of a
-        // launch, where the deepest queries' chains of dependent steps set
-        // the time) takes less time. Every verdict is the conjunction of the
-        // same 15 axes.
+        // 16 W items a lane tests an item's two children, with fewer a lane
+        // tests one child, both through the SAT filter: about 280
+        // instructions a box pair against 900 for the 15 axes as the
+        // reference writes them (DRAM and L2 are idle here; issue and the
+        // dependent latency of a step bound the launch). With an item per
+        // warp or fewer, 16 lanes share a child, an axis each as written (75
+        // instructions), so that the single chains at a launch's start and
+        // end step fastest. Every verdict is the conjunction of the same 15
+        // axes.
         const uint32_t size = top - bot;
-        const uint32_t n = size < 32u ? size : 32u;
+        const uint32_t n = min(size, NT);
         // log2 of lanes per item
-        const uint32_t lg = n <= 1u ? 5u : (n <= 2u ? 4u : (n <= 4u ? 3u : (n <= 8u ? 2u : (n <= 16u ? 1u : 0u))));
-        const uint32_t slot_i = uint32_t(lane) >> lg;
-        const uint32_t sub = uint32_t(lane) & ((1u << lg) - 1u);
+        const uint32_t lg = n <= W ? 5u : (n <= NT / 2u ? 1u : 0u);
+        const uint32_t slot_i = tid >> lg;
+        const uint32_t sub = tid & ((1u << lg) - 1u);
         const bool active = slot_i < n;
         uint32_t iq = 0, is = 0, io = 0;
         if (active) {
@@ -551,41 +524,49 @@ __global__ void __launch_bounds__(256, 2) traverse_kernel(const TraverseParams P
             io = D.b[pos];
         }
         top -= n;
-        __syncwarp();
+        __syncthreads();  // the popped places are rewritten below
+        if (tid == 0) sh.push[par ^ 1u] = 0u;
 
-        // Per lane, per child k: a new item (split node, other record, query
+        // Per lane, per child: a new item (split node, other record, query
         // word) or a candidate leaf pair (triangle offsets and counts).
-        bool item[2] = {false, false}, leaf[2] = {false, false};
-        uint32_t out_q[2] = {0, 0}, out_s[2] = {0, 0}, out_o[2] = {0, 0};
+        Out out0{kNone, 0u, 0u, 0u}, out1 = out0;
         const uint32_t qi = iq & ~kItemSideB;
         const bool sideB = (iq & kItemSideB) != 0;
-        if (lg == 0u) {
+        if (lg <= 1u) {
             if (active) {
                 const Mat4 M = load_mat(P.q + qi);
+                const uint32_t first = is + sub;  // the lane's (first) child
                 const Rec O = load_rec(P.recs, io);
-                const Rec C0 = load_rec(P.recs, is);
-                const Rec C1 = load_rec(P.recs, is + 1u);
-                Box a0, a1, b0, b1;
-                if (sideB) {
-                    a0 = O.box;
-                    a1 = O.box;
-                    b0 = xform_box(M, C0.box);
-                    b1 = xform_box(M, C1.box);
+                const Rec C0 = load_rec(P.recs, first);
+                const Box moved = xform_box(M, sideB ? C0.box : O.box);
+                const SatBox so = sat_box(sideB ? O.box : moved);
+                const Box cb0 = sideB ? moved : C0.box;
+                unsigned open0 = 0, open1 = 0;
+                float err0, err1;
+                if (lg == 0u) {
+                    const Rec C1 = load_rec(P.recs, first + 1u);
+                    Box cb1 = C1.box;
+                    if (sideB) cb1 = xform_box(M, C1.box);
+                    const SatBox s0 = sat_box(cb0), s1 = sat_box(cb1);
+                    bool ok0 = !sat_filter(so, s0, open0);
+                    bool ok1 = !sat_filter(so, s1, open1);
+                    const float surf0 = sat_surface(sideB ? s0 : so, err0);
+                    const float surf1 = sat_surface(sideB ? s1 : so, err1);
+                    if (ok0 && open0) ok0 = overlap_on_axes(so.b, cb0, open0);
+                    if (ok1 && open1) ok1 = overlap_on_axes(so.b, cb1, open1);
+                    out0 = descend(P, ok0, sideB, O, C0, first, io, qi, sideB ? cb0 : so.b, surf0, err0);
+                    out1 = descend(P, ok1, sideB, O, C1, first + 1u, io, qi, sideB ? cb1 : so.b, surf1, err1);
                 } else {
-                    a0 = C0.box;
-                    a1 = C1.box;
-                    b0 = xform_box(M, O.box);
-                    b1 = b0;
+                    const SatBox s0 = sat_box(cb0);
+                    bool ok0 = !sat_filter(so, s0, open0);
+                    const float surf0 = sat_surface(sideB ? s0 : so, err0);
+                    if (ok0 && open0) ok0 = overlap_on_axes(so.b, cb0, open0);
+                    out0 = descend(P, ok0, sideB, O, C0, first, io, qi, sideB ? cb0 : so.b, surf0, err0);
                 }
-                bool ok[2] = {true, true};
-                sat_two(a0, b0, a1, b1, ok[0], ok[1]);
-                if (ok[0]) descend(P, sideB, O, C0, is, io, qi, b0, item[0], leaf[0], out_q[0], out_s[0], out_o[0]);
-                if (ok[1]) descend(P, sideB, O, C1, is + 1u, io, qi, b1, item[1], leaf[1], out_q[1], out_s[1], out_o[1]);
             }
         } else {
-            const uint32_t lc = lg - 1u;               // log2 of lanes per child
-            const uint32_t kc = sub >> lc;             // the child this lane tests
-            const uint32_t ax0 = sub & ((1u << lc) - 1u);  // its first axis; it takes every (1 << lc)-th
+            const uint32_t kc = sub >> 4;   // the child this lane tests
+            const uint32_t ax = sub & 15u;  // its axis
             bool ok = true;
             Rec O, C;
             Box bx;
@@ -593,118 +574,115 @@ __global__ void __launch_bounds__(256, 2) traverse_kernel(const TraverseParams P
                 const Mat4 M = load_mat(P.q + qi);
                 O = load_rec(P.recs, io);
                 C = load_rec(P.recs, is + kc);
-                const Box ax = sideB ? O.box : C.box;
                 bx = xform_box(M, sideB ? C.box : O.box);
-#pragma unroll 1
-                for (uint32_t k = ax0; k < 15u && ok; k += 1u << lc) ok = sat_axis(ax, bx, k);
+                if (ax < 15u) ok = sat_axis(sideB ? O.box : C.box, bx, ax);
             }
-            // the child's verdict: no lane of its group found a separating axis
+            // the child's verdict: none of its 16 lanes found a separating axis
             const unsigned fail = __ballot_sync(kFull, !ok);
-            const unsigned group = (lc == 4u ? 0xffffu : ((1u << (1u << lc)) - 1u)) << (uint32_t(lane) & ~((1u << lc) - 1u));
-            ok = (fail & group) == 0u;
-            if (active && ok && ax0 == 0u)
-                descend(P, sideB, O, C, is + kc, io, qi, bx, item[0], leaf[0], out_q[0], out_s[0], out_o[0]);
+            ok = (fail & (0xffffu << (lane & 16u))) == 0u;
+            if (active && ax == 0u)
+                out0 = descend(P, ok, sideB, O, C, is + kc, io, qi, bx, 0.0f, __int_as_float(0x7f800000));
         }
 
-        const unsigned i0 = __ballot_sync(kFull, item[0]), i1 = __ballot_sync(kFull, item[1]);
-        {
+        // pushes: the warp's places from one shared counter, the lanes' by ballot
+        const unsigned i0 = __ballot_sync(kFull, out0.what == kItem), i1 = __ballot_sync(kFull, out1.what == kItem);
+        const unsigned l0 = __ballot_sync(kFull, out0.what == kLeaf), l1 = __ballot_sync(kFull, out1.what == kLeaf);
+        if (i0 | i1 | l0 | l1) {
+            unsigned off = 0;
+            if (lane == 0)
+                off = atomicAdd(&sh.push[par], (__popc(i0) + __popc(i1)) | (__popc(l0) + __popc(l1)) << 16);
+            off = __shfl_sync(kFull, off, 0);
             const unsigned lt = lanemask_lt();
-            uint32_t r = __popc(i0 & lt) + __popc(i1 & lt);
+            uint32_t r = top + (off & 0xffffu) + __popc(i0 & lt) + __popc(i1 & lt);
+            uint32_t l = nl + (off >> 16) + __popc(l0 & lt) + __popc(l1 & lt);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                if (item[k]) {
-                    const uint32_t p = (top + r) & D.mask;
-                    D.q[p] = out_q[k];
-                    D.a[p] = out_s[k];
-                    D.b[p] = out_o[k];
+                const Out& out = k ? out1 : out0;
+                if (out.what == kItem) {
+                    const uint32_t p = r & D.mask;
+                    D.q[p] = out.q;
+                    D.a[p] = out.s;
+                    D.b[p] = out.o;
                     ++r;
+                }
+                if (out.what == kLeaf) {
+                    lq[l] = qi;
+                    loa[l] = out.s;
+                    lob[l] = out.o;
+                    lcn[l] = out.q;
+                    ++l;
                 }
             }
         }
-        top += __popc(i0) + __popc(i1);
-
-        const unsigned l0 = __ballot_sync(kFull, leaf[0]), l1 = __ballot_sync(kFull, leaf[1]);
-        {
-            const unsigned lt = lanemask_lt();
-            uint32_t r = nl + __popc(l0 & lt) + __popc(l1 & lt);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (leaf[k]) {
-                    lq[r] = qi;
-                    loa[r] = out_s[k];
-                    lob[r] = out_o[k];
-                    lcn[r] = out_q[k];
-                    ++r;
-                }
-            }
-        }
-        nl += __popc(l0) + __popc(l1);
-        if (lane == 0) {
+        if (tid == 0) {
+            sh.qs[par] = qs;
             st_nodes += 2u * n;
-            ++st_steps;
+            st_steps += ((n << lg) + 31u) >> 5;  // steps of warps that hold items
             if (P.trace) trace_add(P.trace, P.trace_ns, t_base, 0, n);
         }
-        __syncwarp();
+        __syncthreads();
+        const unsigned pushed = sh.push[par];
+        top += pushed & 0xffffu;
+        nl += pushed >> 16;
+        qs = sh.qs[par];
+        par ^= 1u;
 
-        if (nl >= P.leaf_flush) {
-            flush_leafs(P, lq, loa, lob, lcn, nl, lane);
+        if (nl > (P.leaf_flush - 1u) * W) {
+            flush_leafs(P, sh, lq, loa, lob, lcn, nl);
             nl = 0;
         }
 
-        // ---- balance: give chunks from the bottom of the deque to the warps
-        // that wait (one chunk per waiting warp, up to 8, keeping at least a
-        // chunk; a full chunk when the deque is nearly full). A warp does not
-        // take queued chunks while it has work: that costs a contended atomic
-        // per step and measured slower.
+        // ---- balance: give chunks from the bottom of the deque to the blocks
+        // that wait (one chunk per waiting block, keeping at least a chunk; a
+        // full chunk when the deque is nearly full). A block does not take
+        // queued chunks while it has work: that costs a contended atomic per
+        // step and measured slower.
         const uint32_t held = top - bot;
-        const bool forced = held + 64u > S;
-        int mode = 0;  // 1: donate nch chunks of c
-        uint32_t c = 0, nch = 0, slot = 0;
-        if (lane == 0) {
-            const int waiting = int(ht_head(qs) - ht_tail(qs));
-            if (forced || (waiting > 0 && held >= P.donate_min)) {
-                c = held >= 2u * kChunk ? uint32_t(kChunk) : (held >> 1);
-                nch = min(uint32_t(waiting > 0 ? waiting : 1), min(held / c - 1u, 8u));
-                if (nch == 0) nch = 1;
-                if (ht_tail(qs) - P.n_queries + nch <= P.slot_cap) {
-                    slot = ht_tail(atomicAdd(ht, (unsigned long long)nch << 32));
+        const bool forced = held + 64u * W > S;
+        const int waiting = int(ht_head(qs) - ht_tail(qs));
+        if (forced || (waiting > 0 && held >= P.donate_min)) {
+            const uint32_t c = held >= 2u * kChunk ? uint32_t(kChunk) : (held >> 1);
+            const uint32_t want = max(uint32_t(max(waiting, 1)), forced ? W : 1u);
+            const uint32_t nch = max(1u, min(want, min(held / c - 1u, 8u * W)));
+            if (tid == 0) {
+                int mode = 0;
+                if (ht_tail(qs) + nch <= P.slot_cap) {
+                    sh.slot = ht_tail(atomicAdd(ht, (unsigned long long)nch << 32));
                     mode = 1;
                 } else if (forced) {
                     atomicOr(&P.ctr->error, ERR_QUEUE);
                     mode = -1;
                 }
+                sh.mode = mode;
             }
-        }
-        mode = __shfl_sync(kFull, mode, 0);
-        if (mode == -1) break;
-        if (mode == 1) {
-            c = __shfl_sync(kFull, c, 0);
-            nch = __shfl_sync(kFull, nch, 0);
-            slot = __shfl_sync(kFull, slot, 0);
-            const uint32_t idx0 = slot - P.n_queries;
-            for (uint32_t ch = 0; ch < nch; ++ch) {
-                if (uint32_t(lane) < c) {
-                    const uint32_t pos = (bot + ch * c + lane) & D.mask;
-                    P.pool[size_t(kChunk) * (idx0 + ch) + lane] = make_uint4(D.q[pos], D.a[pos], D.b[pos], 0u);
+            __syncthreads();
+            if (sh.mode == -1) break;
+            if (sh.mode == 1) {
+                const uint32_t slot = sh.slot;
+                for (uint32_t k = tid; k < nch * c; k += NT) {
+                    const uint32_t ch = k / c, pos = (bot + k) & D.mask;
+                    P.pool[size_t(kChunk) * (slot + ch) + (k - ch * c)] = make_uint4(D.q[pos], D.a[pos], D.b[pos], 0u);
                 }
+                __threadfence();
+                __syncthreads();
+                for (uint32_t k = tid; k < nch; k += NT) st_release(P.ready + slot + k, c + 1u);
+                if (tid == 0) st_don += c * nch;
+                bot += c * nch;
             }
-            __threadfence();
-            __syncwarp();
-            if (uint32_t(lane) < nch) st_release(P.ready + idx0 + lane, c + 1u);
-            if (lane == 0) st_don += c * nch;
-            bot += c * nch;
-            __syncwarp();
         }
 
         if (top == bot) {
-            if (lane == 0) atomicAdd(&P.ctr->done, held_tasks);
+            // every thread has read the shared words of this step's end
+            __syncthreads();
+            if (tid == 0) atomicAdd(&P.ctr->done, held_tasks);
             held_tasks = 0;
         }
     }
 
     // remaining buffered leaf pairs
-    if (nl) flush_leafs(P, lq, loa, lob, lcn, nl, lane);
-    if (lane == 0) {
+    __syncthreads();
+    if (nl) flush_leafs(P, sh, lq, loa, lob, lcn, nl);
+    if (tid == 0) {
         if (st_nodes) atomicAdd(&P.ctr->node_pairs, st_nodes);
         if (st_don) atomicAdd(&P.ctr->donations, st_don);
         if (st_steps) atomicAdd(&P.ctr->warp_steps, st_steps);
@@ -812,11 +790,7 @@ __global__ void pack_kernel(const cg_query* in, uint32_t n, const DevTree* trees
 __global__ void init_kernel(Counters* ctr, unsigned int* ready, uint32_t slot_alloc, uint32_t n_queries,
                             unsigned int* trace) {
     __shared__ uint32_t used;
-    if (threadIdx.x == 0) {
-        const uint32_t tail = ctr->tail;
-        const uint32_t prev_n = ctr->n_queries;
-        used = tail > prev_n ? min(tail - prev_n, slot_alloc) : 0u;
-    }
+    if (threadIdx.x == 0) used = min(ctr->tail, slot_alloc);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < used; i += blockDim.x) ready[i] = 0u;
     if (trace)
@@ -824,7 +798,6 @@ __global__ void init_kernel(Counters* ctr, unsigned int* ready, uint32_t slot_al
     __syncthreads();
     if (threadIdx.x == 0) {
         Counters c = {};
-        c.tail = n_queries;
         c.n_queries = n_queries;
         // vertex-set slots stay taken until a contacts launch empties them
         c.prev_vertices = ctr->prev_vertices + ctr->n_vertices;
@@ -865,21 +838,56 @@ cudaError_t launch_surfaces(float4* recs, uint32_t first, uint32_t n_recs, cudaS
     return cudaGetLastError();
 }
 
+namespace {
+// Warps of a worker block. Two: a worker's steps are wide enough to advance a
+// query's whole frontier in most of them, and an SM holds four workers that
+// hide one another's latency; a launch of at most one query per eight warps
+// has no other work for them, and four warps widen the step further.
+// Traversal alone, 1, 2, 4 and 8 warps (us): 1 query of 2 x 2,048 triangles
+// 59, 51, 48, 47; 64 of these 85, 67, 58, 64; 150 queries of 2 x 20,000 213,
+// 180, 190, 202; the 256-entity scene 131, 103, 110, 119; 10,000 uneven
+// queries 1310, 1288, 1392, 1587.
+uint32_t worker_warps(uint32_t n_queries, uint32_t total_warps) {
+    return uint64_t(n_queries) * 8u <= total_warps && total_warps >= 4u ? 4u : (total_warps >= 2u ? 2u : 1u);
+}
+constexpr uint32_t kStackMax = 4096;  // cg_config.stack_entries' limit
+}  // namespace
+
 cudaError_t traverse_occupancy(uint32_t warps_per_block, uint32_t stack_cap, int* blocks_per_sm) {
-    const size_t smem = size_t(warps_per_block) * warp_smem_words(stack_cap) * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute(traverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    // the widest worker's deque at the largest stack: one limit for every
+    // context of the process
+    cudaError_t e = cudaFuncSetAttribute(traverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(traverse_smem_words(kStackMax, 4u) * sizeof(uint32_t)));
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, traverse_kernel, int(32 * warps_per_block),
-                                                         smem);
+    int device = 0, limit = 0, two = 0, four = 0;
+    if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) != cudaSuccess) return e;
+    *blocks_per_sm = 0;
+    // a setting whose warps' stacks together are more than a block may hold
+    if (size_t(warps_per_block) * (3u * stack_cap + 4u * kLeafCap) * sizeof(uint32_t) > size_t(limit))
+        return cudaSuccess;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, traverse_kernel, 64,
+                                                      traverse_smem_words(stack_cap, 2u) * sizeof(uint32_t));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&four, traverse_kernel, 128,
+                                                          traverse_smem_words(stack_cap, 4u) * sizeof(uint32_t));
+    const int warps = std::min(2 * two, 4 * four);
+    *blocks_per_sm = warps ? std::max(1, warps / int(warps_per_block)) : 0;
+    return e;
 }
 
 cudaError_t narrow_occupancy(uint32_t warps_per_block, int* blocks_per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, narrow_kernel<0>, int(32 * warps_per_block), 0);
 }
 
-cudaError_t launch_traverse(const TraverseParams& p, uint32_t blocks, uint32_t warps_per_block, cudaStream_t s) {
-    const size_t smem = size_t(warps_per_block) * warp_smem_words(p.stack_cap) * sizeof(uint32_t);
-    traverse_kernel<<<blocks, 32 * warps_per_block, smem, s>>>(p);
+cudaError_t launch_traverse(const TraverseParams& p_in, uint32_t blocks, uint32_t warps_per_block, cudaStream_t s) {
+    TraverseParams p = p_in;
+    const uint32_t total = blocks * warps_per_block, W = worker_warps(p.n_queries, total), workers = total / W;
+    p.donate_min *= W;
+    // all roots start at once where they fit a step of the workers
+    p.root_batch = std::min(std::max((p.n_queries + workers - 1u) / workers, 1u), 32u * W);
+    const size_t smem = size_t(traverse_smem_words(p.stack_cap, W)) * sizeof(uint32_t);
+    traverse_kernel<<<workers, 32 * W, smem, s>>>(p);
     return cudaGetLastError();
 }
 
