@@ -277,6 +277,7 @@ int alloc_buffers(cg_ctx* c) {
     CG_CUDA(contacts_fold_occupancy(&focc), "occupancy");
     c->fold_blocks = uint32_t(std::max(focc, 1) * c->sm_count);
     CG_CUDA(deform_smem_limit(), "deform kernel shared memory");
+    CG_CUDA(build_smem_limit(), "build kernel shared memory");
     c->copy_blocks = uint32_t(4 * c->sm_count);
     int gocc = 0;
     CG_CUDA(energy_occupancy(&gocc), "occupancy");

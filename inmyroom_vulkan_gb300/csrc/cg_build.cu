@@ -17,8 +17,8 @@
 //   build_terms   a thread per triangle position: the six centred products
 //                 of its corners
 //   build_cov     a thread per node and product: the covariance sum in
-//                 corner order (build_cov_big: a warp per node of more
-//                 than kBuildBig triangles)
+//                 corner order (build_cov_big: a block per product of a node
+//                 of more than kBuildBig triangles)
 //   build_eig     a thread per node: eig3 of the covariance in FP64; the
 //                 box axes are the rows of the eigenvector matrix
 //   build_proj    a thread per triangle position: its corners' FP64
@@ -51,6 +51,7 @@
 // the device (build_gather) before the first level.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -59,6 +60,7 @@
 #include "cg_device.cuh"
 #include "cg_eig.cuh"
 #include "cg_internal.h"
+#include "cg_replay.cuh"
 
 namespace cg {
 
@@ -449,17 +451,230 @@ __global__ void build_cov_kernel(const BuildParams B) {
     }
 }
 
-// The same for the list's nodes of more than kBuildBig triangles, a
-// one-warp block each (lanes 0-5 its six chains): a large node's chains
-// share their warp's FP64 instructions and loads with no other node's.
-__global__ void __launch_bounds__(32) build_cov_big_kernel(const BuildParams B) {
+// Long sums in parallel segments (cg_replay.cuh), a block per sum, a tile of
+// kTile terms in shared memory at a time:
+//   sums of 8 terms by a thread each and their prefix sum give the predicted
+//   sum at every 8th term; each run of kSegment terms starts a segment at
+//   its sample of the largest magnitude (so that the states after it lie at
+//   most a binade above it), unless the next four runs hold sums more than a
+//   binade larger; 4 candidates of each segment run side by side, a lane each;
+//   then one thread links the segments from the true sum at the tile's start.
+// Per term about a fifth of a warp's FP64 add instead of one, and 8,192 terms
+// in 25 to 50 us instead of 300 (a chain's 76 cycles a term): bound by the
+// segments' chains and their linking. The covariances of nodes of more than
+// 256 triangles, all levels: of a 5,003-triangle mesh 1,337 to 381 us, of 256
+// meshes (1.4 M triangles) 6.2 to 3.5 ms. The coordinate sums (floats, whose
+// running sums rarely round) stay with the exact integer counts above, which
+// are faster for them.
+constexpr uint32_t kSample = 8, kSegment = 64;
+
+// The block of a tile of kTile terms: four samples a thread, four lanes for
+// every two runs.
+template <uint32_t kTile>
+struct Replay {
+    static constexpr uint32_t kThreads = kTile / (4u * kSample), kSamples = kTile / kSample, kRuns = kTile / kSegment;
+    static_assert(kThreads % 32u == 0u, "whole warps");
+    double t[kTile + kTile / 16u];      // the tile's terms; one place in 17 unused (banks)
+    double sum[kSamples];               // predicted sum before every 8th term
+    double warp[kThreads / 32u];
+    uint32_t peak[kRuns];               // a run's largest and first sums' exponent fields; then its segment's start
+    uint32_t start[kRuns + 1u];         // the segments' first samples
+    double pred[kRuns + 1u];            // their predicted sums
+    uint32_t n_seg;
+    ReplayLink end[4u * kRuns];
+    double total;                       // predicted sum after the tile
+    double s;
+};
+// Two sizes: a tile of 8,192 terms for nodes of more than kReplayMid
+// triangles, and 2,048 with 64 threads (ten blocks an SM) for smaller ones.
+using ReplayBig = Replay<8192>;
+using ReplayMid = Replay<2048>;
+constexpr uint32_t kReplayMid = 1024;
+
+__device__ __forceinline__ uint32_t tile_at(uint32_t j) { return j + (j >> 4); }
+
+// The sum of x[0..n-1] in order, from +0; all threads of the block, each gets
+// it.
+template <uint32_t kTile>
+__device__ double replay_sum(const double* __restrict__ x, uint32_t n, Replay<kTile>& R) {
+    constexpr uint32_t kReplayThreads = Replay<kTile>::kThreads;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    double s = 0.0;
+    for (uint32_t base = 0; base < n; base += kTile) {
+        const uint32_t m = min(kTile, n - base);
+        // the last sample filled up with -0, which no sum is changed by
+        for (uint32_t j = tid; j < (m + kSample - 1u) / kSample * kSample; j += kReplayThreads)
+            R.t[tile_at(j)] = j < m ? x[base + j] : -0.0;
+        __syncthreads();
+        // predicted sums: thread i's four samples
+        double h[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            const uint32_t j0 = (4u * tid + k) * kSample;
+            if (j0 < m) {
+#pragma unroll
+                for (uint32_t j = 0; j < kSample; ++j) h[k] = h[k] + R.t[tile_at(j0 + j)];
+            }
+        }
+        const double half = h[0] + h[1], all = half + (h[2] + h[3]);
+        double inc = all;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double u = __shfl_up_sync(kAll, inc, o);
+            if (lane >= uint32_t(o)) inc = inc + u;
+        }
+        if (lane == 31u) R.warp[w] = inc;
+        __syncthreads();
+        if (w == 0u) {  // the sums before each warp
+            constexpr uint32_t kWarps = kReplayThreads / 32u;
+            double v = lane < kWarps ? R.warp[lane] : 0.0;
+            const double own = v;
+#pragma unroll
+            for (uint32_t o = 1; o < kWarps; o <<= 1) {
+                const double u = __shfl_up_sync(kAll, v, o);
+                if (lane >= o) v = v + u;
+            }
+            if (lane < kWarps) R.warp[lane] = s + (v - own);
+        }
+        __syncthreads();
+        const double before = tid ? R.warp[w] + (inc - all) : s;  // the tile's start is the true sum
+        R.sum[4u * tid] = before;
+        R.sum[4u * tid + 1u] = before + h[0];
+        R.sum[4u * tid + 2u] = before + half;
+        R.sum[4u * tid + 3u] = before + (half + h[2]);
+        if (tid + 1u == kReplayThreads) R.total = before + all;
+        __syncthreads();
+        // each run's largest sum and its first one
+        constexpr uint32_t kPer = kSegment / kSample;
+        const uint32_t runs = (m + kSegment - 1u) / kSegment, samples = (m + kSample - 1u) / kSample;
+        auto exponent = [&](uint32_t k) { return uint32_t(dbits(R.sum[k]) >> 52) & 0x7ffu; };
+        for (uint32_t r = tid; r < runs; r += kReplayThreads) {
+            uint32_t best = 0;
+            for (uint32_t k = r * kPer; k < min(samples, (r + 1u) * kPer); ++k)
+                best = max(best, uint32_t(dbits(R.sum[k]) >> 32) & 0x7fffffffu);
+            // a sum between two samples may be somewhat larger than both
+            R.peak[r] = (best + 0x20000u) >> 20 | exponent(r * kPer) << 16;
+        }
+        __syncthreads();
+        // the segments, from the last run to the first: a run starts one at its
+        // first sample if no sum up to the next segment is more than a binade
+        // above that (every 16th run does in any case, which bounds a
+        // segment's length)
+        if (tid == 0u) {
+            uint32_t top = 0;
+#pragma unroll 4
+            for (uint32_t r = runs; r-- > 0u;) {
+                const uint32_t p = R.peak[r];
+                top = max(top, p & 0xffffu);
+                const bool keep = (p >> 16) + 1u >= top || (r & 15u) == 0u;
+                R.peak[r] = keep ? r * kPer : 0xffffffffu;
+                top = keep ? 0u : top;
+            }
+        }
+        __syncthreads();
+        if (w == 0u) {
+            uint32_t count = 0;
+            for (uint32_t r0 = 0; r0 < runs; r0 += 32u) {
+                const uint32_t r = r0 + lane;
+                const uint32_t at = r < runs ? R.peak[r] : 0xffffffffu;
+                const unsigned b = __ballot_sync(kAll, at != 0xffffffffu);
+                if (at != 0xffffffffu) {
+                    const uint32_t g = count + __popc(b & ((1u << lane) - 1u));
+                    R.start[g] = at;
+                    R.pred[g] = R.sum[at];
+                }
+                count += __popc(b);
+            }
+            if (lane == 0u) {
+                R.start[count] = samples;
+                R.pred[count] = R.total;
+                R.n_seg = count;
+            }
+        }
+        __syncthreads();
+        // the candidates: four lanes take every (threads / 4)-th segment, all
+        // lanes of a warp in one loop over samples, so that a warp's time is
+        // its lanes' longest total; the adds are the chain, the next terms'
+        // loads and the last states' checks run beside them
+        const uint32_t n_seg = R.n_seg, first = tid & 3u;
+        uint32_t g = tid >> 2, at = 0, to = 0;
+        double v = 0.0, start = 0.0;
+        ReplayChain seen;
+        bool busy = g < n_seg;
+        if (busy) {
+            start = v = replay_candidate(R.pred[g], first);
+            at = R.start[g], to = R.start[g + 1u];
+        }
+        double term[kSample];
+#pragma unroll
+        for (uint32_t j = 0; j < kSample; ++j) term[j] = R.t[tile_at(at * kSample + j)];
+        while (__any_sync(kAll, busy)) {
+            ++at;
+            const bool ends = at >= to;
+            const uint32_t from = (ends ? at - 1u : at) * kSample;  // the next sample's place
+            double ahead[kSample];
+#pragma unroll
+            for (uint32_t j = 0; j < kSample; ++j) {
+                const double last = v;
+                v = v + term[j];
+                ahead[j] = R.t[tile_at(from + j)];
+                replay_see(seen, last);
+            }
+            if (busy && ends) {
+                replay_see(seen, v);
+                R.end[4u * g + first] = replay_end(start, seen, v, R.pred[g + 1u]);
+                g += kReplayThreads / 4u;
+                busy = g < n_seg;
+                if (busy) {
+                    start = v = replay_candidate(R.pred[g], first);
+                    at = R.start[g], to = R.start[g + 1u];
+                    seen = ReplayChain{};
+#pragma unroll
+                    for (uint32_t j = 0; j < kSample; ++j) ahead[j] = R.t[tile_at(at * kSample + j)];
+                } else {
+                    at = to = 0u;  // idle: sample 0 again
+                }
+            }
+            if (!busy) at = 0u;
+#pragma unroll
+            for (uint32_t j = 0; j < kSample; ++j) term[j] = ahead[j];
+        }
+        __syncthreads();
+        if (tid == 0u) {
+            const double v = replay_chain(s, R.pred, R.end, n_seg, [&](uint32_t g, double u) {
+                const uint32_t j1 = R.start[g + 1u] * kSample;
+#pragma unroll 8
+                for (uint32_t j = R.start[g] * kSample; j < j1; ++j) u = u + R.t[tile_at(j)];
+                return u;
+            });
+            R.s = v;
+        }
+        __syncthreads();
+        s = R.s;
+    }
+    return s;
+}
+
+// Whether a node of more than kBuildBig triangles is this tile size's.
+template <class R>
+__device__ __forceinline__ bool replays(uint32_t count) {
+    return (count > kReplayMid) == (R::kThreads == ReplayBig::kThreads);
+}
+
+// The same for the level's nodes of more than kBuildBig triangles, a block
+// per product.
+template <class R>
+__global__ void __launch_bounds__(R::kThreads) build_cov_big_kernel(const BuildParams B) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    R& sh = *reinterpret_cast<R*>(smem);
     const uint64_t n3 = 3ull * B.T;
-    const uint32_t q = threadIdx.x;
-    if (q >= 6u) return;
-    for (uint32_t i = blockIdx.x; i < B.n_big; i += gridDim.x) {
-        const uint32_t id = B.big[i];
+    for (uint32_t i = blockIdx.x; i < 6u * B.n_big; i += gridDim.x) {
+        const uint32_t id = B.big[i / 6u], q = i % 6u;
         const BuildNode& N = B.nodes[id];
-        B.mom[9ull * (id - B.lo) + 3u + q] = chain_sum(B.Tm + q * n3 + 3ull * N.begin, 3u * N.count);
+        if (!replays<R>(N.count)) continue;
+        const double s = replay_sum(B.Tm + q * n3 + 3ull * N.begin, 3u * N.count, sh);
+        if (threadIdx.x == 0u) B.mom[9ull * (id - B.lo) + 3u + q] = s;
+        __syncthreads();
     }
 }
 
@@ -1124,6 +1339,11 @@ __global__ void build_emit_tris_kernel(const BuildParams B, const BuildInput I, 
 
 }  // namespace
 
+cudaError_t build_smem_limit() {
+    return cudaFuncSetAttribute(build_cov_big_kernel<ReplayBig>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(sizeof(ReplayBig)));
+}
+
 cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStream_t s) {
     if (p.hi <= p.lo) return cudaSuccess;
     const uint32_t width = p.hi - p.lo;
@@ -1134,13 +1354,18 @@ cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStre
     };
     build_points_kernel<<<grid(p.T), 128, 0, s>>>(p);
     build_sums_kernel<<<grid(3ull * width), 128, 0, s>>>(p);
+    const uint32_t most = 65535u;
     if (p.n_big) {
-        build_sums_big_kernel<<<p.n_big < 65535u ? p.n_big : 65535u, kBigWarps * 32u, 0, s>>>(p);
+        build_sums_big_kernel<<<std::min(p.n_big, most), kBigWarps * 32u, 0, s>>>(p);
         build_sums_due_kernel<<<grid(3ull * p.n_big), 128, 0, s>>>(p);
     }
     build_terms_kernel<<<grid(p.T), 128, 0, s>>>(p);
     build_cov_kernel<<<grid(6ull * width), 128, 0, s>>>(p);
-    if (p.n_big) build_cov_big_kernel<<<p.n_big < 65535u ? p.n_big : 65535u, 32, 0, s>>>(p);
+    if (p.n_big) {
+        const uint32_t g = std::min(6u * p.n_big, most);
+        build_cov_big_kernel<ReplayBig><<<g, ReplayBig::kThreads, sizeof(ReplayBig), s>>>(p);
+        build_cov_big_kernel<ReplayMid><<<g, ReplayMid::kThreads, sizeof(ReplayMid), s>>>(p);
+    }
     build_eig_kernel<<<grid(width), 128, 0, s>>>(p);
     build_proj_kernel<<<grid(p.T), 128, 0, s>>>(p);
     if (p.n_big) build_fit_big_kernel<<<p.n_big < 65535u ? p.n_big : 65535u, kBigWarps * 32u, 0, s>>>(p);

@@ -478,6 +478,7 @@ struct BuildParams {
     uint32_t* n_big_out;
 };
 constexpr uint32_t kBuildBig = 256;  // nodes of more than this many triangles are fitted by a block
+cudaError_t build_smem_limit();
 cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStream_t s);
 struct BuildMesh {
     uint32_t vbase;          // first vertex in BuildInput::vertices / normals
