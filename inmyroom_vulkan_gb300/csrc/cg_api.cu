@@ -54,8 +54,10 @@ void free_buffers(cg_ctx* c) {
     cudaFree(c->d_ready);
     cudaFree(c->d_pairs);
     cudaFree(c->d_leafs);
-    cudaFree(c->d_leaf_keys);
-    c->d_leaf_keys = nullptr;
+    for (void* p : {(void*)c->order.keys, (void*)c->order.key[0], (void*)c->order.key[1], (void*)c->order.place,
+                    (void*)c->order.index[0], (void*)c->order.index[1], (void*)c->order.queries})
+        cudaFree(p);
+    c->order = cg_ctx::LeafOrder{};
     cudaFree(c->d_trace);
     auto& t = c->ct;
     for (void* p : {(void*)t.pair_aux, (void*)t.table, (void*)t.occupied, (void*)t.slot_info, (void*)t.big_slots, (void*)t.pg_geom, (void*)t.pg_link,
@@ -419,7 +421,8 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
     np.pairs_cap = c->d_pairs ? c->cfg.max_tri_pairs : 0;
     np.leafs = c->d_leafs;
     np.leafs_cap = c->d_leafs ? c->cfg.max_leaf_pairs : 0;
-    np.flags = flags;
+    // ordered leaf pairs are written by the ordering kernels
+    np.flags = (flags & CG_DFS_ORDER) ? flags & ~CG_KEEP_LEAF_PAIRS : flags;
     np.trace = trace;
     np.trace_ns = trace_ns;
     const unsigned rec_flags = c->capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -437,8 +440,25 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
         kp.n_leafs = &c->d_ctr->n_leafs;
         kp.leaf_cap = p.leaf_cap;
         kp.error = &c->d_ctr->error;
-        kp.keys = c->d_leaf_keys;
+        kp.keys = c->order.keys;
+        kp.count = c->order.queries;
+        kp.place = c->order.place;
+        CG_CUDA(cudaMemsetAsync(kp.count, 0, sizeof(uint32_t) * n, s), "clear leaf-pair counts");
         CG_CUDA(launch_leaf_keys(kp, c->contact_blocks, s), "leaf-pair key kernel");
+        LeafOrderParams op{};
+        op.q = c->d_packed;
+        op.n_queries = n;
+        op.leaf_list = c->d_leaf_list;
+        op.n_leafs = kp.n_leafs;
+        op.leaf_cap = p.leaf_cap;
+        op.keys = kp.keys;
+        op.count = kp.count;
+        op.place = kp.place;
+        op.first = kp.count + c->cfg.max_queries;
+        op.tile = op.first + c->cfg.max_queries;
+        for (int k = 0; k < 2; ++k) op.key[k] = c->order.key[k], op.index[k] = c->order.index[k];
+        op.out = c->d_leafs;
+        CG_CUDA(launch_leaf_order(op, uint32_t(c->sm_count), s), "leaf-pair order kernels");
     }
     if (pairs_copy) {
         CG_CUDA(cudaEventRecord(c->ev_fork, s), "fork event");
@@ -563,8 +583,17 @@ int check_flags(cg_ctx* c, uint32_t flags) {
         if (!(flags & CG_KEEP_LEAF_PAIRS) || !c->d_leafs)
             return fail(c, CG_ERR_INVALID_ARGUMENT, "CG_DFS_ORDER orders the kept leaf pairs: it needs "
                         "CG_KEEP_LEAF_PAIRS and max_leaf_pairs > 0");
-        if (!c->d_leaf_keys)
-            CG_CUDA(cudaMalloc(&c->d_leaf_keys, sizeof(ulonglong2) * c->cfg.max_leaf_pairs), "alloc leaf-pair keys");
+        auto& o = c->order;
+        const uint64_t m = c->cfg.max_leaf_pairs;
+        if (!o.queries) {
+            if (!o.keys) CG_CUDA(cudaMalloc(&o.keys, sizeof(ulonglong2) * m), "alloc leaf-pair keys");
+            if (!o.place) CG_CUDA(cudaMalloc(&o.place, sizeof(uint32_t) * m), "alloc leaf-pair places");
+            for (int k = 0; k < 2; ++k) {
+                if (!o.key[k]) CG_CUDA(cudaMalloc(&o.key[k], sizeof(ulonglong2) * m), "alloc leaf-pair order");
+                if (!o.index[k]) CG_CUDA(cudaMalloc(&o.index[k], sizeof(uint32_t) * m), "alloc leaf-pair order");
+            }
+            CG_CUDA(cudaMalloc(&o.queries, sizeof(uint32_t) * (3ull * c->cfg.max_queries + 1u)), "alloc leaf-pair order");
+        }
     }
     if (!(flags & CG_CONTACTS)) return CG_OK;
     if (!c->cfg.max_contacts) return fail(c, CG_ERR_INVALID_ARGUMENT, "CG_CONTACTS needs max_contacts > 0");
@@ -1115,23 +1144,7 @@ int cg_read_leaf_pairs(cg_ctx* c, cg_leaf_pair* out, uint64_t cap, uint64_t* n) 
     const uint64_t avail = std::min<uint64_t>(c->h_ctr->n_leafs, c->d_leafs ? c->cfg.max_leaf_pairs : 0);
     *n = c->h_ctr->n_leafs;
     const uint64_t m = std::min(avail, cap);
-    if (m && (c->last_flags & CG_DFS_ORDER)) {
-        // grouped by query, each query's in the order of its descent path
-        std::vector<cg_leaf_pair> all(avail);
-        std::vector<ulonglong2> keys(avail);
-        CG_CUDA(cudaMemcpy(all.data(), c->d_leafs, sizeof(cg_leaf_pair) * avail, cudaMemcpyDeviceToHost),
-                "read leaf pairs");
-        CG_CUDA(cudaMemcpy(keys.data(), c->d_leaf_keys, sizeof(ulonglong2) * avail, cudaMemcpyDeviceToHost),
-                "read leaf-pair keys");
-        std::vector<uint32_t> order(avail);
-        for (uint32_t i = 0; i < avail; ++i) order[i] = i;
-        std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-            if (all[x].query != all[y].query) return all[x].query < all[y].query;
-            if (keys[x].x != keys[y].x) return keys[x].x < keys[y].x;
-            return keys[x].y < keys[y].y;
-        });
-        for (uint64_t i = 0; i < m; ++i) out[i] = all[order[i]];
-    } else if (m) {
+    if (m) {
         CG_CUDA(cudaMemcpy(out, c->d_leafs, sizeof(cg_leaf_pair) * m, cudaMemcpyDeviceToHost), "read leaf pairs");
     }
     return c->h_ctr->n_leafs > avail ? CG_ERR_OUTPUT_OVERFLOW : CG_OK;

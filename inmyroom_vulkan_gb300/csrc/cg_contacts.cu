@@ -1730,6 +1730,7 @@ __global__ void __launch_bounds__(kPathWarps * 32) leaf_keys_kernel(const LeafKe
         if (!(lane & 1u) && valid) {
             if (depth >= 128u) atomicOr(P.error, ERR_DEEP);
             P.keys[i] = make_ulonglong2(hi, lo);
+            P.place[i] = atomicAdd(P.count + lp.x, 1u);
         }
         __syncwarp();
     }

@@ -139,7 +139,12 @@ struct cg_ctx {
     uint4* d_leaf_list = nullptr;   // candidate leaf pairs between the two kernels
     cg_tri_pair* d_pairs = nullptr;
     cg_leaf_pair* d_leafs = nullptr;
-    ulonglong2* d_leaf_keys = nullptr;  // CG_DFS_ORDER: each leaf pair's descent path (allocated on first use)
+    // CG_DFS_ORDER, allocated on first use: each leaf pair's descent path and
+    // number within its query, the sort's two buffers, the queries' counts and places
+    struct LeafOrder {
+        ulonglong2 *keys = nullptr, *key[2] = {nullptr, nullptr};
+        uint32_t *place = nullptr, *index[2] = {nullptr, nullptr}, *queries = nullptr;
+    } order;
     unsigned int* d_trace = nullptr;
     uint32_t trace_ns = 0;
 

@@ -209,8 +209,28 @@ struct LeafKeyParams {
     uint32_t leaf_cap;
     unsigned* error;                    // ERR_DEEP when a path is too deep for 128 bits
     ulonglong2* keys;                   // per leaf pair: path high, low
+    uint32_t* count;                    // per query: its leaf pairs (zero before the launch)
+    uint32_t* place;                    // per leaf pair: its number within its query
 };
 cudaError_t launch_leaf_keys(const LeafKeyParams& p, uint32_t grid, cudaStream_t s);
+
+// The leaf pairs grouped by query and sorted by path (cg_leaf_order.cu).
+struct LeafOrderParams {
+    const PackedQuery* q;
+    uint32_t n_queries;
+    const uint4* leaf_list;
+    const unsigned long long* n_leafs;
+    uint32_t leaf_cap;
+    const ulonglong2* keys;   // launch_leaf_keys' results
+    const uint32_t* count;
+    const uint32_t* place;
+    uint32_t* first;          // [n_queries] scratch: each query's first place
+    uint32_t* tile;           // [n_queries + 1] scratch: its first tile
+    ulonglong2* key[2];       // [leaf_cap] scratch
+    uint32_t* index[2];
+    cg_leaf_pair* out;
+};
+cudaError_t launch_leaf_order(const LeafOrderParams& p, uint32_t sm_count, cudaStream_t s);
 
 // Results of a step written to host buffers (cg_set_host_outputs).
 struct CopyOutParams {
