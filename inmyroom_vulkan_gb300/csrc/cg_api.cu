@@ -524,7 +524,8 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
             cp.sched_start[k] = c->sched_start[k];
             cp.sched_buckets[k] = c->sched_buckets[k];
         }
-        CG_CUDA(launch_contacts(cp, c->contact_blocks, c->fold_blocks, c->order_blocks, s, c->branch,
+        CG_CUDA(launch_contacts(cp, c->contact_blocks, c->fold_blocks, c->order_blocks,
+                                uint32_t(c->sm_count), s, c->branch,
                                 c->ev_branch, c->ev_branched), "contact kernels");
     }
     if (pairs_copy) CG_CUDA(cudaStreamWaitEvent(s, c->ev_joined, 0), "join");

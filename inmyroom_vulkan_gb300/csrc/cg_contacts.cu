@@ -562,30 +562,26 @@ __device__ __forceinline__ void k_keep(K& x, const K& y, bool keep_min) {
     if (K::less(y, x) == keep_min) x = y;
 }
 
-constexpr uint32_t kSortThreads = 256;               // the order kernel's block
-constexpr uint32_t kRegSortMax = 4u * kSortThreads;  // keys the block sorts in registers
-
-// Ascending bitonic sort by the block (kSortThreads threads) of n2 keys (a
-// power of two, 32 <= n2 <= E * kSortThreads, E = 1, 2 or 4); thread t holds
-// keys t + 256 e: exchanges within a warp by shuffles, across warps through
-// xchg (n2 keys of shared memory, two barriers), between a thread's own keys
-// in registers.
-template <class K, int E>
+// Ascending bitonic sort by the block (T threads) of n2 keys (a power of two,
+// 32 <= n2 <= E * T, E = 1, 2 or 4); thread t holds keys t + T e: exchanges
+// within a warp by shuffles, across warps through xchg (n2 keys of shared
+// memory, two barriers), between a thread's own keys in registers.
+template <uint32_t T, class K, int E>
 __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg) {
     const uint32_t t = threadIdx.x;
     const bool active = t < n2;  // warp-uniform: n2 is a multiple of 32
     for (uint32_t k = 2; k <= n2; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            if (j >= kSortThreads) {
-                // a thread's own keys e and e ^ (j / 256); the lower one keeps
+            if (j >= T) {
+                // a thread's own keys e and e ^ (j / T); the lower one keeps
                 // the minimum when ascending
-                const uint32_t jj = j / kSortThreads;
+                const uint32_t jj = j / T;
 #pragma unroll
                 for (int e = 0; e < E; ++e)
 #pragma unroll
                     for (int f = e + 1; f < E; ++f)
                         if (uint32_t(e ^ f) == jj) {
-                            const bool asc = ((t + kSortThreads * uint32_t(e)) & k) == 0u;
+                            const bool asc = ((t + T * uint32_t(e)) & k) == 0u;
                             const K lo = x[e], hi = x[f];
                             const bool sw = K::less(hi, lo) == asc;
                             x[e] = sw ? hi : lo;
@@ -594,13 +590,13 @@ __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg)
             } else if (j >= 32u) {
                 if (active) {
 #pragma unroll
-                    for (int e = 0; e < E; ++e) xchg[t + kSortThreads * e] = x[e];
+                    for (int e = 0; e < E; ++e) xchg[t + T * e] = x[e];
                 }
                 __syncthreads();
                 if (active) {
 #pragma unroll
                     for (int e = 0; e < E; ++e) {
-                        const uint32_t i = t + kSortThreads * e;
+                        const uint32_t i = t + T * e;
                         k_keep(x[e], xchg[i ^ j], ((i & j) == 0u) == ((i & k) == 0u));
                     }
                 }
@@ -608,7 +604,7 @@ __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg)
             } else if (active) {
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
-                    const uint32_t i = t + kSortThreads * e;
+                    const uint32_t i = t + T * e;
                     k_keep(x[e], x[e].xor_lane(j), ((i & j) == 0u) == ((i & k) == 0u));
                 }
             }
@@ -617,22 +613,22 @@ __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg)
 }
 
 // The insertion order of the map's n elements El (n2 = pow2 >= max(n, 32),
-// n2 <= E * kSortThreads): keys from the elements' paths and triangles,
+// n2 <= E * T): keys from the elements' paths and triangles,
 // sorted, then per insertion index its triangle and element.
-template <class K, int E>
+template <uint32_t T, class K, int E>
 __device__ __forceinline__ void insertion_order(const ContactElem* El, uint32_t n, uint32_t n2, void* xchg,
                                                 uint32_t* ins_tri, uint32_t* ins_elem) {
     const uint32_t t = threadIdx.x;
     K x[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const uint32_t i = t + kSortThreads * e;
+        const uint32_t i = t + T * e;
         x[e] = i < n ? K::make(El[i].key_hi, El[i].key_lo, El[i].tri, i) : K::pad();
     }
-    block_sort_regs<K, E>(x, n2, reinterpret_cast<K*>(xchg));
+    block_sort_regs<T, K, E>(x, n2, reinterpret_cast<K*>(xchg));
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const uint32_t i = t + kSortThreads * e;
+        const uint32_t i = t + T * e;
         if (i < n) {
             ins_tri[i] = x[e].tri();
             ins_elem[i] = x[e].elem();
@@ -1059,6 +1055,7 @@ __device__ void rank_maps(const ContactParams& P) {
         for (int c = 32; c >= 0; --c) {
             start[c] = off;
             off += count[c];
+            if (1u << (c > 0 ? c - 1 : 0) == kBigMap) P.ctr->n_bigmaps = off;
         }
     }
     __syncthreads();
@@ -1082,14 +1079,14 @@ __device__ void place_maps(const ContactParams& P, uint32_t* part) {
     }
 }
 
-// True in the block that finishes last of the grid (counted on `done`); its
+// True in the block that finishes last of `blocks` (counted on `done`); its
 // threads then see every other block's writes.
-__device__ bool last_block(unsigned* done) {
+__device__ bool last_block(unsigned* done, uint32_t blocks) {
     __shared__ bool last;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        last = atomicAdd(done, 1u) == gridDim.x - 1u;
+        last = atomicAdd(done, 1u) == blocks - 1u;
     }
     __syncthreads();
     if (last) __threadfence();
@@ -1131,7 +1128,7 @@ __global__ void __launch_bounds__(256, 3) contacts_fold_kernel(const ContactPara
         fold_warp(P, key, si.z, si.w, stage[wib], F);
         if (lane == 0) put_elem(P, key, F);
     }
-    if (last_block(&P.ctr->fold_done)) rank_maps(P);
+    if (last_block(&P.ctr->fold_done, gridDim.x)) rank_maps(P);
 }
 
 // A ray of find_rays_lambda (CreateUncollideRays.cpp:140-173) for contact
@@ -1194,25 +1191,24 @@ __device__ cg_ray contact_ray(const ContactParams& P, uint32_t q, uint32_t side,
 // The vertex set of one map (CreateUncollideRays.cpp:148-161, the
 // emplaced_point_indices set): each vertex index of a corner that may make a
 // ray, with the place code (place * 4 + corner) of its first such corner in
-// iteration order. In shared memory (keys: vertex indices, ~0u empty; `mask`
-// + 1 slots, a power of two, hashed by the top bits of a multiplicative
-// hash) when `keys` is set, else the launch's global set keyed by (side,
-// query, vertex index).
+// iteration order. In shared memory (keys: vertex indices, ~0u empty; `slots`
+// of them, a multiplicative hash scaled to that range) when `keys` is set,
+// else the launch's global set keyed by (side, query, vertex index).
 struct VSet {
     uint32_t* keys;
     uint32_t* vals;
-    uint32_t mask, shift;
+    uint32_t slots;
 };
 
 __device__ __forceinline__ int smem_insert(const VSet& V, uint32_t key, uint32_t* slot) {
-    uint32_t s = (key * 0x9E3779B1u) >> V.shift;
-    for (uint32_t probe = 0; probe <= V.mask; ++probe) {
+    uint32_t s = __umulhi(key * 0x9E3779B1u, V.slots);
+    for (uint32_t probe = 0; probe < V.slots; ++probe) {
         const uint32_t cur = atomicCAS(V.keys + s, ~0u, key);
         if (cur == ~0u || cur == key) {
             *slot = s;
             return cur == ~0u ? 1 : 0;
         }
-        s = (s + 1u) & V.mask;
+        if (++s == V.slots) s = 0u;
     }
     return -1;
 }
@@ -1300,25 +1296,26 @@ __device__ void warp_steps(const ContactParams& P, uint32_t n, uint32_t steps, c
     }
 }
 
-// One map (query, side) by the whole block: its triangles in the reference's
-// iteration order, their contact records and rays in that order, and the
-// map's mean ray origin.
+// One map (query, side) by the whole block (T threads, kWords words of shared
+// memory): its triangles in the reference's iteration order, their contact
+// records and rays in that order, and the map's mean ray origin.
+template <uint32_t T, uint32_t kWords>
 __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, uint32_t* part, float* fold) {
     const uint32_t q = map >> 1, side = map & 1u;
     const uint32_t n = P.map_fill[map];
     const uint32_t base = P.map_off[map];
-    const uint32_t T = blockDim.x, t = threadIdx.x;
+    const uint32_t t = threadIdx.x;
     uint32_t n_rays = 0;
     bool ok = n > 0u && base + n <= P.max_contacts;
     OrderLayout L{};
     uint32_t* W = smem;
-    VSet V{nullptr, nullptr, 0u, 0u};
+    VSet V{nullptr, nullptr, 0u};
     if (ok) {
         L = order_layout(P, n);
-        // the vertex set: at most 3 n keys, at most three quarters full
-        const uint32_t hs = pow2_ceil(4u * n);
-        uint32_t used = L.words;
-        if (L.words + 2u * hs > kOrderSmemWords) {
+        // the vertex set (at most 3 n keys, often half that) takes what the
+        // ray phase leaves of the shared memory, four slots a triangle at most
+        uint32_t used = 10u * L.nr;
+        if (L.words > kWords) {
             // this map's part of the global working memory: kOrderWords per
             // element from its first element (base + n <= max_contacts)
             W = P.work + size_t(kOrderWords) * base;
@@ -1326,15 +1323,11 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
             if (!ok && t == 0u) atomicOr(&P.ctr->c_overflow, CONTACT_ORDER);
             used = 0u;
         }
-        if (used + 2u * hs <= kOrderSmemWords) {
+        const uint32_t slots = min(4u * n, (kWords - used) / 2u);
+        if (slots >= 3u * n + n / 4u) {
             V.keys = smem + used;
-            V.vals = V.keys + hs;
-            V.mask = hs - 1u;
-            V.shift = 33u - uint32_t(__ffs(hs));
-            for (uint32_t i = t; i < hs; i += T) {
-                V.keys[i] = ~0u;
-                V.vals[i] = ~0u;
-            }
+            V.vals = V.keys + slots;
+            V.slots = slots;
         }
     }
     cg_ray* R = P.rtmp + 3ull * base;
@@ -1347,7 +1340,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
         uint32_t* mask_of = W + 2u * L.nr;
         uint32_t* B0 = W + 3u * L.nr;
         // 1. insertion order: the first leaf pair's path, then the triangle
-        if (L.n2 <= kRegSortMax) {
+        if (L.n2 <= 4u * T) {
             bool wide = false, mid = false;  // a path with low-word bits; with bits in the high word's low half
             for (uint32_t i = t; i < n; i += T) {
                 const ContactElem& E = El[i];
@@ -1357,19 +1350,20 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
             }
             wide = __syncthreads_or(wide) != 0;
             mid = __syncthreads_or(mid) != 0;
-            const uint32_t E = L.n2 <= kSortThreads ? 1u : (L.n2 <= 2u * kSortThreads ? 2u : 4u);
+            const uint32_t E = L.n2 <= T ? 1u : (L.n2 <= 2u * T ? 2u : 4u);
+            uint32_t* xchg = W == smem ? B0 : smem;  // 6 n2 words at most
             if (!wide && !mid) {
-                if (E == 1u) insertion_order<K1, 1>(El, n, L.n2, B0, ins_tri, ins_elem);
-                else if (E == 2u) insertion_order<K1, 2>(El, n, L.n2, B0, ins_tri, ins_elem);
-                else insertion_order<K1, 4>(El, n, L.n2, B0, ins_tri, ins_elem);
+                if (E == 1u) insertion_order<T, K1, 1>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                else if (E == 2u) insertion_order<T, K1, 2>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                else insertion_order<T, K1, 4>(El, n, L.n2, xchg, ins_tri, ins_elem);
             } else if (!wide) {
-                if (E == 1u) insertion_order<K2, 1>(El, n, L.n2, B0, ins_tri, ins_elem);
-                else if (E == 2u) insertion_order<K2, 2>(El, n, L.n2, B0, ins_tri, ins_elem);
-                else insertion_order<K2, 4>(El, n, L.n2, B0, ins_tri, ins_elem);
+                if (E == 1u) insertion_order<T, K2, 1>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                else if (E == 2u) insertion_order<T, K2, 2>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                else insertion_order<T, K2, 4>(El, n, L.n2, xchg, ins_tri, ins_elem);
             } else {
-                if (E == 1u) insertion_order<K3, 1>(El, n, L.n2, B0, ins_tri, ins_elem);
-                else if (E == 2u) insertion_order<K3, 2>(El, n, L.n2, B0, ins_tri, ins_elem);
-                else insertion_order<K3, 4>(El, n, L.n2, B0, ins_tri, ins_elem);
+                if (E == 1u) insertion_order<T, K3, 1>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                else if (E == 2u) insertion_order<T, K3, 2>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                else insertion_order<T, K3, 4>(El, n, L.n2, xchg, ins_tri, ins_elem);
             }
         } else {
             SortKey* sk = reinterpret_cast<SortKey*>(B0);
@@ -1475,6 +1469,13 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
         // 3. rays: the vertex set keeps each vertex index's first corner. Per
         // place: mask then vertex-ray corners (rb), rays (rc), its corners'
         // vertex indices (vi0..2); the order stays where the last step left it
+        if (V.keys) {
+            for (uint32_t i = t; i < V.slots; i += T) {
+                V.keys[i] = ~0u;
+                V.vals[i] = ~0u;
+            }
+            __syncthreads();
+        }
         uint32_t* rb = B0 + 2u * L.nr;
         uint32_t* rc = B0 + 3u * L.nr;
         uint32_t* vi0 = B0 + 4u * L.nr;
@@ -1553,7 +1554,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
     // the mean origin: std::accumulate over the rays in order, one coordinate
     // per lane, from shared memory a chunk of rays at a time
     {
-        constexpr uint32_t kStageRays = kOrderSmemWords / 3u;
+        constexpr uint32_t kStageRays = kWords / 3u;
         float* stage = reinterpret_cast<float*>(smem);
         float acc = 0.0f;
         for (uint32_t r0 = 0; r0 < n_rays; r0 += kStageRays) {
@@ -1595,25 +1596,34 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
     }
 }
 
-// Persistent: each block takes the next map of the largest-first list.
-__global__ void __launch_bounds__(256, 2) contacts_order_kernel(const ContactParams P) {
+// Persistent: each block takes the next map of the largest-first list. Two
+// launches side by side (the second a programmatic dependent of the first: a
+// branch of its own cost one-query steps 4 us): the maps of kBigMap triangles or more by blocks of
+// 1,024 threads with an SM's whole shared memory, the others by blocks of 256.
+// The block that finishes last of both places the maps.
+template <uint32_t T, uint32_t kWords, bool kBig>
+__global__ void __launch_bounds__(T, kBig ? 1 : 2) contacts_order_kernel(const ContactParams P) {
     extern __shared__ __align__(16) uint32_t smem_order[];
     __shared__ uint32_t part[64];
     __shared__ float fold[3];
     __shared__ uint32_t next_map;
-    const uint32_t n_maps = 2u * P.n_queries;
+    // the small maps' launch may start beside this one, and ends after it
+    if (kBig) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t big = *reinterpret_cast<const volatile unsigned*>(&P.ctr->n_bigmaps);
+    const uint32_t end = kBig ? big : 2u * P.n_queries;
     for (;;) {
         if (threadIdx.x == 0) {
-            const uint32_t i = atomicAdd(&P.ctr->order_ticket, 1u);
-            next_map = i < n_maps ? P.map_order[i] : ~0u;
+            const uint32_t i = kBig ? atomicAdd(&P.ctr->order_big_ticket, 1u) : big + atomicAdd(&P.ctr->order_ticket, 1u);
+            next_map = i < end ? P.map_order[i] : ~0u;
         }
         __syncthreads();
         const uint32_t map = next_map;
         if (map == ~0u) break;
-        order_map(P, map, smem_order, part, fold);
+        order_map<T, kWords>(P, map, smem_order, part, fold);
         __syncthreads();
     }
-    if (last_block(&P.ctr->order_done)) place_maps(P, part);
+    if (!kBig) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (last_block(&P.ctr->order_done, P.order_grid)) place_maps(P, part);
 }
 
 __global__ void __launch_bounds__(256) contacts_emit_kernel(const ContactParams P) {
@@ -1741,19 +1751,29 @@ cudaError_t launch_leaf_keys(const LeafKeyParams& p, uint32_t grid, cudaStream_t
     return cudaGetLastError();
 }
 
+namespace {
+constexpr auto order_small = contacts_order_kernel<256, kOrderSmemWords, false>;
+constexpr auto order_big = contacts_order_kernel<1024, kBigSmemWords, true>;
+}  // namespace
+
 cudaError_t contacts_order_occupancy(int* blocks_per_sm) {
     const int smem = int(kOrderSmemWords * sizeof(uint32_t));
-    cudaError_t e = cudaFuncSetAttribute(contacts_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(order_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(order_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kBigSmemWords * sizeof(uint32_t)));
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, contacts_order_kernel, 256, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, order_small, 256, smem);
 }
 
 cudaError_t contacts_fold_occupancy(int* blocks_per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, contacts_fold_kernel, 256, 0);
 }
 
-cudaError_t launch_contacts(const ContactParams& p, uint32_t grid, uint32_t fold_grid, uint32_t order_grid,
-                            cudaStream_t s, cudaStream_t branch, cudaEvent_t ev_fork, cudaEvent_t ev_join) {
+cudaError_t launch_contacts(const ContactParams& p_in, uint32_t grid, uint32_t fold_grid, uint32_t order_grid,
+                            uint32_t big_grid, cudaStream_t s, cudaStream_t branch, cudaEvent_t ev_fork,
+                            cudaEvent_t ev_join) {
+    ContactParams p = p_in;
     if (!p.n_queries) return cudaSuccess;
     const uint32_t maps = 2u * p.n_queries;
     contacts_pairs_kernel<<<grid, 256, 0, s>>>(p);
@@ -1770,7 +1790,20 @@ cudaError_t launch_contacts(const ContactParams& p, uint32_t grid, uint32_t fold
     e = cudaStreamWaitEvent(s, ev_join, 0);
     if (e != cudaSuccess) return e;
     contacts_fold_kernel<<<fold_grid, 256, 0, s>>>(p);
-    contacts_order_kernel<<<maps < order_grid ? maps : order_grid, 256, kOrderSmemWords * sizeof(uint32_t), s>>>(p);
+    const uint32_t small = maps < order_grid ? maps : order_grid, big = maps < big_grid ? maps : big_grid;
+    p.order_grid = small + big;
+    order_big<<<big, 1024, kBigSmemWords * sizeof(uint32_t), s>>>(p);
+    cudaLaunchAttribute beside{};
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(small);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = kOrderSmemWords * sizeof(uint32_t);
+    cfg.stream = s;
+    cfg.attrs = &beside;
+    cfg.numAttrs = 1;
+    if ((e = cudaLaunchKernelEx(&cfg, order_small, p)) != cudaSuccess) return e;
     contacts_emit_kernel<<<maps < grid ? maps : grid, 256, 0, s>>>(p);
     return cudaGetLastError();
 }

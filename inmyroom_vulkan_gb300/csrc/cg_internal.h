@@ -96,7 +96,9 @@ struct Counters {
     unsigned int prev_vertices;  // vertex-set slots earlier launches took and no launch emptied yet
     unsigned int n_kleaf;        // leaf pairs with colliding pairs (listed for their descent paths)
     unsigned int contrib_used;   // contribution-list entries given to slots
-    unsigned int order_ticket;   // maps taken by the order kernel's blocks
+    unsigned int order_ticket;   // maps of fewer than kBigMap triangles taken by the order kernel's blocks
+    unsigned int order_big_ticket;  // larger maps taken
+    unsigned int n_bigmaps;      // larger maps
     unsigned int n_big;          // contact slots of more than kFoldThread contributions (listed for the fold)
     unsigned int fold_done;      // fold blocks finished (the last one ranks the maps)
     unsigned int order_done;     // order blocks finished (the last one places the maps' records and rays)
@@ -133,11 +135,15 @@ struct alignas(16) ContactElem {
 // buckets[e] (the whole table is rehashed into it when start[e] is inserted).
 constexpr uint32_t kMaxSchedule = 40;
 
-// Order kernel working memory: a map whose working set and vertex set fit
-// kOrderSmemWords words (every map of up to 1,024 triangles) is ordered in
-// shared memory, larger ones in global memory (kOrderWords words per
-// element).
+// Order kernel working memory: maps of fewer than kBigMap triangles are
+// ordered in kOrderSmemWords words of shared memory (two blocks an SM), larger
+// ones in kBigSmemWords (a block an SM) where their working set fits (up to
+// about 3,500 triangles), else in global memory (kOrderWords words per
+// element). The line lies where a map stops fitting half an SM: a map of 1,500
+// triangles took 530,000 cycles in global memory with 256 threads.
+constexpr uint32_t kBigMap = 1024;
 constexpr uint32_t kOrderSmemWords = 24576;
+constexpr uint32_t kBigSmemWords = 57344;
 constexpr uint32_t kOrderWords = 24;
 constexpr uint32_t kFoldThread = 8;  // contributions a slot's own thread folds (more: its warp)
 
@@ -192,10 +198,11 @@ struct ContactParams {
     Counters* ctr;
     uint32_t sched_start[kMaxSchedule];
     uint32_t sched_buckets[kMaxSchedule];
+    uint32_t order_grid;        // blocks of both order launches
 };
 
 cudaError_t launch_contacts(const ContactParams& p, uint32_t grid, uint32_t fold_grid, uint32_t order_grid,
-                            cudaStream_t s, cudaStream_t branch, cudaEvent_t ev_fork, cudaEvent_t ev_join);
+                            uint32_t big_grid, cudaStream_t s, cudaStream_t branch, cudaEvent_t ev_fork, cudaEvent_t ev_join);
 cudaError_t contacts_order_occupancy(int* blocks_per_sm);
 cudaError_t contacts_fold_occupancy(int* blocks_per_sm);
 
