@@ -529,6 +529,14 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
                                 c->ev_branch, c->ev_branched), "contact kernels");
     }
     if (pairs_copy) CG_CUDA(cudaStreamWaitEvent(s, c->ev_joined, 0), "join");
+    // a captured step (here or by the caller) may be replayed without a call:
+    // it leaves its counters on the host itself
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    CG_CUDA(cudaStreamIsCapturing(s, &st), "capture status");
+    if (st == cudaStreamCaptureStatusNone)
+        c->ctr_mirrored = false;
+    else
+        CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s), "copy counters");
     return CG_OK;
 }
 
@@ -577,6 +585,18 @@ int stats_from(cg_ctx* c, const Counters& k, cg_stats* st) {
     s.status = status;
     if (st) *st = s;
     return status;
+}
+
+// The last launch's counters in c->h_ctr, once the stream's work is done. A
+// step that cg_collide or a captured graph runs copies them there itself
+// (another round trip took 10 us of every read); else they are copied here.
+int fetch_counters(cg_ctx* c) {
+    if (!c->ctr_mirrored)
+        CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream),
+                "read counters");
+    CG_CUDA(cudaStreamSynchronize(c->stream), "collide");
+    c->ctr_mirrored = true;
+    return CG_OK;
 }
 
 int check_flags(cg_ctx* c, uint32_t flags) {
@@ -994,7 +1014,10 @@ int cg_tree_free(cg_ctx* c, uint32_t id) {
         cudaFree(s.topo);
     }
     s = cg_ctx::Slot{};
-    return sync_tree_table(c);
+    // the table's entry alone (the whole table took 9 us a call for 256 trees)
+    const uint32_t dead = 0;
+    CG_CUDA(cudaMemcpy(&c->d_trees[id].live, &dead, sizeof(dead), cudaMemcpyHostToDevice), "update tree table");
+    return CG_OK;
 }
 
 int cg_collide_async(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flags, void* stream) {
@@ -1015,8 +1038,8 @@ int cg_collide_async(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t 
 int cg_sync_stats(cg_ctx* c, cg_stats* st) {
     if (!c) return CG_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
-    CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "read counters");
-    CG_CUDA(cudaStreamSynchronize(c->stream), "collide");
+    const int frc = fetch_counters(c);
+    if (frc != CG_OK) return frc;
     return stats_from(c, *c->h_ctr, st);
 }
 
@@ -1069,8 +1092,6 @@ int cg_collide(cg_ctx* c, const cg_query* queries, uint32_t n, uint32_t flags, c
         int rc = e == cudaSuccess ? enqueue_step(c, static_cast<const cg_query*>(q_dev), n, flags, c->stream,
                                                  pc.host_pairs ? &pc : nullptr, &rc2)
                                   : CG_ERR_CUDA;
-        if (rc == CG_OK && e == cudaSuccess)
-            e = cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream);
         c->capturing = false;
         cudaGraph_t g = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
@@ -1087,6 +1108,7 @@ int cg_collide(cg_ctx* c, const cg_query* queries, uint32_t n, uint32_t flags, c
         G.out_gen = c->host_out.gen;
     }
     CG_CUDA(cudaGraphLaunch(G.exec, c->stream), "collide step");
+    c->ctr_mirrored = true;
     CG_CUDA(cudaStreamSynchronize(c->stream), "collide");
     return stats_from(c, *c->h_ctr, st);
 }
@@ -1094,8 +1116,8 @@ int cg_collide(cg_ctx* c, const cg_query* queries, uint32_t n, uint32_t flags, c
 int cg_read_tri_pairs(cg_ctx* c, cg_tri_pair* out, uint64_t cap, uint64_t* n) {
     if (!c || !n || (cap && !out)) return CG_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
-    CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "read counters");
-    CG_CUDA(cudaStreamSynchronize(c->stream), "read counters");
+    const int frc = fetch_counters(c);
+    if (frc != CG_OK) return frc;
     const uint64_t avail = std::min<uint64_t>(c->h_ctr->n_pairs, c->d_pairs ? c->cfg.max_tri_pairs : 0);
     *n = c->h_ctr->n_pairs;
     const uint64_t m = std::min(avail, cap);
@@ -1140,8 +1162,8 @@ int cg_set_host_outputs(cg_ctx* c, cg_tri_pair* pairs, uint64_t pairs_cap, cg_ra
 int cg_read_leaf_pairs(cg_ctx* c, cg_leaf_pair* out, uint64_t cap, uint64_t* n) {
     if (!c || !n || (cap && !out)) return CG_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
-    CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "read counters");
-    CG_CUDA(cudaStreamSynchronize(c->stream), "read counters");
+    const int frc = fetch_counters(c);
+    if (frc != CG_OK) return frc;
     const uint64_t avail = std::min<uint64_t>(c->h_ctr->n_leafs, c->d_leafs ? c->cfg.max_leaf_pairs : 0);
     *n = c->h_ctr->n_leafs;
     const uint64_t m = std::min(avail, cap);
@@ -1156,9 +1178,7 @@ namespace {
 int contact_counters(cg_ctx* c) {
     if (!(c->last_flags & CG_CONTACTS)) return fail(c, CG_ERR_INVALID_ARGUMENT, "the last launch had no CG_CONTACTS");
     cudaSetDevice(c->device);
-    CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "read counters");
-    CG_CUDA(cudaStreamSynchronize(c->stream), "read counters");
-    return CG_OK;
+    return fetch_counters(c);
 }
 }  // namespace
 
@@ -1508,6 +1528,7 @@ int cg_graph_launch(cg_ctx* c, void* stream) {
     cudaSetDevice(c->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->stream;
     CG_CUDA(cudaGraphLaunch(c->graph_exec, s), "graph launch");
+    c->ctr_mirrored = true;
     c->last_flags = c->graph_flags;
     c->last_n = c->graph_n;
     return join_stream(c, s);

@@ -187,6 +187,7 @@ struct cg_ctx {
 
     cg_query* h_queries = nullptr;  // pinned
     Counters* h_ctr = nullptr;      // pinned
+    bool ctr_mirrored = false;      // h_ctr holds the last launch's counters once the stream's work is done
 
     uint32_t last_flags = 0;
     uint32_t last_n = 0;            // queries of the last collide step enqueued
@@ -268,6 +269,7 @@ void put_box(float4* rec, const cg_obb& b, uint32_t ref, uint32_t meta, uint32_t
 int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flags, cudaStream_t s,
                  const CopyOutParams* pairs_copy = nullptr, const CopyOutParams* results_copy = nullptr);
 int stats_from(cg_ctx* c, const Counters& k, cg_stats* st);
+int fetch_counters(cg_ctx* c);
 int check_flags(cg_ctx* c, uint32_t flags);
 int join_stream(cg_ctx* c, cudaStream_t s);
 void mat_mul(const float* A, const float* B, float* R);
