@@ -281,6 +281,49 @@ __device__ __forceinline__ void snap3(float3 a0, float3 a1, float3 a2, float3 e1
         if (!(kMode == 2 && unc[k]) && tiny(d[k])) d[k] = 0.0f;
 }
 
+// A triangle's plane for planes_miss: its normal by FMA, the product of its
+// edges' 1-norms and its largest coordinate magnitude.
+struct TriPlane {
+    float3 n;
+    float l, c;
+};
+__device__ __forceinline__ TriPlane tri_plane(float3 p0, float3 p1, float3 p2) {
+    const float3 a = sub3(p1, p0), b = sub3(p2, p0);
+    TriPlane t;
+    t.n = make_float3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
+    t.l = norm1(a) * norm1(b);
+    t.c = fmaxf(fmaxf(amax3(p0), amax3(p1)), amax3(p2));
+    return t;
+}
+
+// Whether tri_tri_mode certainly answers TT_MISS from one of its two plane
+// tests (every corner of one triangle on one side of the other's plane): the
+// distances by FMA in any order, each side's within half the filter bound of
+// the exact determinant, as the reference's are, so a distance beyond 1e-6 by
+// twice the bound has the reference's sign and is none that the recheck
+// recomputes. The bound's C is taken over all six corners. For the recheck
+// (kMode != 0) the second plane's test counts only where the first one's
+// distances are all sure, so that the rechecked distances are the same.
+// A NaN or an overflow leaves the pair to the whole test.
+template <int kMode>
+__device__ __forceinline__ bool planes_miss(float3 V0, float3 V1, float3 V2, const TriPlane& A, float3 U0, float3 U1,
+                                            float3 U2, const TriPlane& B) {
+    auto dot = [](float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); };
+    // (three comparisons, not a minimum: those drop a NaN)
+    auto beyond = [](float x, float y, float z, float t) {
+        return (x > t && y > t && z > t) || (x < -t && y < -t && z < -t);
+    };
+    const float C = fmaxf(A.c, B.c), lim = 1.0001e-6f, k = 2.5f * kRecheckU32 * C;
+    const float t1 = fmaf(k, A.l, lim), t2 = fmaf(k, B.l, lim);
+    const bool sane = C < 1e10f;
+    const float3 w = sub3(U0, V0);
+    const float du0 = dot(A.n, w), du1 = dot(A.n, sub3(U1, V0)), du2 = dot(A.n, sub3(U2, V0));
+    if (sane && beyond(du0, du1, du2, t1)) return true;
+    const float dv0 = -dot(B.n, w), dv1 = dot(B.n, sub3(V1, U0)), dv2 = dot(B.n, sub3(V2, U0));
+    const bool sure = kMode == 0 || (fabsf(du0) > t1 && fabsf(du1) > t1 && fabsf(du2) > t1);
+    return sane && sure && beyond(dv0, dv1, dv2, t2);
+}
+
 // tri_tri_intersect_with_isectline (Triangle.cpp:866-1003). TT_HIT means
 // doIntersept && !areCoplanar (the pairs CreateUncollideRays.cpp:88 keeps);
 // TT_COPLANAR covers every coplanar outcome (never kept); TT_FRAGILE is the
