@@ -503,6 +503,7 @@ struct BuildParams {
     uint32_t n_big;
     uint32_t* big_out;       // the next level's, appended by the splits of this level's
     uint32_t* n_big_out;
+    bool early;              // the next kernel's blocks may start beside this one
 };
 constexpr uint32_t kBuildBig = 256;  // nodes of more than this many triangles are fitted by a block
 cudaError_t build_smem_limit();
