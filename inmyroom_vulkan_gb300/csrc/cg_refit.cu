@@ -242,7 +242,8 @@ __device__ __forceinline__ float unkey(int k) { return __int_as_float(k >= 0 ? k
 // every box above it. Leaves are in tree order, so a warp's leaves share most
 // of their chains. Bound by the latency of each level's loads and by issue: at
 // six blocks an SM (80 registers), by FMA and without the reductions that move
-// nothing, the refit of 64 trees of 12,000 triangles takes 327 us (351 before).
+// nothing, the refit of 64 trees of 12,000 triangles takes 327 us (351 before;
+// 300 with the axes' eigensystems in registers, too).
 __global__ void __launch_bounds__(128, 6) refit_extent_kernel(const float4* tris, const RefitTree* trees,
                                                            const RefitBufs B) {
     const RefitTree T = trees[blockIdx.y];
