@@ -76,9 +76,10 @@ int cg_tree_build(cg_ctx* c, const cg_mesh_view* meshes, uint32_t n, uint32_t* t
     const size_t oNodes = take(sizeof(BuildNode) * cap), oFlat = take(sizeof(BuildFlat) * cap),
                  oCtr = take(sizeof(LevelState));
     const size_t oSegs = take(sizeof(PullSeg) * 3 * n);
-    // a level's nodes of more than kBuildBig triangles: the roots, or disjoint
-    // ranges of more than kBuildBig triangles each
-    const uint64_t big_cap = n + T / (kBuildBig + 1) + 1;
+    // a level's nodes of more than big_min triangles: the roots, or disjoint
+    // ranges of more than big_min triangles each
+    const uint32_t big_min = build_big_min(T, uint32_t(c->sm_count));
+    const uint64_t big_cap = n + T / (big_min + 1) + 1;
     const size_t oBig = take(sizeof(uint32_t) * 2 * big_cap);
     const size_t oV = take(sizeof(float) * 3 * std::max<uint64_t>(nv, 1));
     const size_t oNV = take(any_normals ? sizeof(float) * 3 * std::max<uint64_t>(nv, 1) : 0);
@@ -113,6 +114,7 @@ int cg_tree_build(cg_ctx* c, const cg_mesh_view* meshes, uint32_t n, uint32_t* t
     bp.error = bp.node_ctr + 1;
     in.bad = reinterpret_cast<unsigned long long*>(mem + oCtr + offsetof(LevelState, bad));
     bp.node_cap = cap;
+    bp.big_min = big_min;
     bp.T = uint32_t(total);
     uint32_t* big_list[2] = {reinterpret_cast<uint32_t*>(mem + oBig), reinterpret_cast<uint32_t*>(mem + oBig) + big_cap};
     float* d_V = reinterpret_cast<float*>(mem + oV);
@@ -172,7 +174,7 @@ int cg_tree_build(cg_ctx* c, const cg_mesh_view* meshes, uint32_t n, uint32_t* t
     const LevelState st0{{n, 0u, 0u, 0u}, ~0ull};
     std::vector<uint32_t> big_roots;
     for (uint32_t i = 0; i < n; ++i)
-        if (roots[i].count > kBuildBig) big_roots.push_back(i);
+        if (roots[i].count > big_min) big_roots.push_back(i);
     CG_CUDA(cudaMemcpyAsync(d_mesh, mt.data(), sizeof(BuildMesh) * n, cudaMemcpyHostToDevice, s), "upload meshes");
     CG_CUDA(cudaMemcpyAsync(bp.nodes, roots.data(), sizeof(BuildNode) * n, cudaMemcpyHostToDevice, s), "upload roots");
     CG_CUDA(cudaMemcpyAsync(bp.node_ctr, &st0, sizeof(st0), cudaMemcpyHostToDevice, s), "upload counter");

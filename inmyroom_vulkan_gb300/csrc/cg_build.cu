@@ -13,20 +13,21 @@
 // chains runs a thread per corner on every SM:
 //   build_points  a thread per triangle position: its corners as doubles
 //   build_sums    a thread per node and coordinate: the sum in corner order,
-//                 the mean
+//                 the mean (build_sums_mid, build_sums_big: blocks for a
+//                 node of more than big_min triangles)
 //   build_terms   a thread per triangle position: the six centred products
 //                 of its corners
 //   build_cov     a thread per node and product: the covariance sum in
 //                 corner order (build_cov_big: a block per product of a node
-//                 of more than kBuildBig triangles)
+//                 of more than big_min triangles)
 //   build_eig     a thread per node: eig3 of the covariance in FP64; the
 //                 box axes are the rows of the eigenvector matrix
 //   build_proj    a thread per triangle position: its corners' FP64
 //                 projections on its node's axes
-//   build_fit     a warp per node of more than 16 triangles (build_fit_small:
-//                 a thread per smaller node; build_fit_big: a block per node
-//                 of more than kBuildBig): fewer than two distinct corners
-//                 give the empty or point box; else the min/max projections
+//   build_fit     a warp per node (build_fit_small: a thread per node of at
+//                 most 16 triangles of a wide level; build_fit_big: a block
+//                 per node of more than big_min): fewer than two distinct
+//                 corners give the empty or point box; else the min/max projections
 //                 (integer keys of the doubles; equal values: the later
 //                 corner, as the sequential std::min / std::max keep) and the
 //                 box; then, for a node of more than 4 triangles,
@@ -68,7 +69,7 @@ namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
 constexpr uint32_t kLeafMax = 4;  // OBBtree.h:49 maxNumberOfTriangles
-constexpr uint32_t kBigWarps = 16;  // warps of the block that handles one node of more than kBuildBig triangles
+constexpr uint32_t kBigWarps = 16;  // warps of the block that handles one node of more than big_min triangles
 
 __device__ __forceinline__ float3 corner(const float* P, uint32_t t, uint32_t k) {
     const float* q = P + 9ull * t + 3u * k;
@@ -235,7 +236,7 @@ __global__ void build_sums_kernel(const BuildParams B) {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         const uint32_t node = B.lo + g / 3u, c = g % 3u;
         const BuildNode& N = B.nodes[node];
-        if (N.count > kBuildBig) continue;  // build_sums_big
+        if (N.count > B.big_min) continue;  // build_sums_mid, build_sums_big
         const uint32_t np = 3u * N.count;
         const double s = chain_sum(B.D + c * n3 + 3ull * N.begin, np);
         B.mom[9ull * (node - B.lo) + c] = np ? s / double(np) : 0.0;
@@ -305,8 +306,17 @@ __device__ __forceinline__ long long round_double(long long count) {
 constexpr uint32_t kSumChunk = 32;   // consecutive terms a thread adds up at a time
 constexpr uint32_t kSumRounds = 64;  // roundings replayed before a sum is left to the chain
 
-// A block per node of the level's list of nodes of more than kBuildBig
-// triangles: the coordinate sums of build_sums_kernel without the chain. The
+// Nodes of the level's list of few triangles whose coordinate sums are
+// replayed in segments, too (build_sums_mid): up to 1,024 triangles that is
+// faster than the integer counts, whose passes take 37 us even for a few
+// hundred triangles (segments: 15), where there is room for it.
+constexpr uint32_t kReplayMid = 1024;
+__device__ __forceinline__ bool replays_sums(const BuildParams& B, uint32_t count) {
+    return count <= kReplayMid && B.big_min == kBuildBigFew;
+}
+
+// A block per node of the level's list of nodes of more than big_min
+// triangles (replays_sums' apart): the coordinate sums of build_sums_kernel without the chain. The
 // terms are floats, integer multiples of 2^q (q the smallest exponent of
 // their ulps), so the sequential sum is replayed exactly in 64-bit integer
 // counts of 2^q (the terms are bounded so that no running sum can overflow):
@@ -329,6 +339,7 @@ __global__ void __launch_bounds__(kBigWarps * 32) build_sums_big_kernel(const Bu
     for (uint32_t i = blockIdx.x; i < B.n_big; i += gridDim.x) {
         const uint32_t id = B.big[i];
         const BuildNode& N = B.nodes[id];
+        if (replays_sums(B, N.count)) continue;
         const uint32_t np = 3u * N.count;
         const double* x0 = B.D + 3ull * N.begin;
         // the smallest ulp exponent and the largest exponent of the non-zero terms
@@ -484,7 +495,7 @@ __global__ void build_cov_kernel(const BuildParams B) {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         const uint32_t node = B.lo + g / 6u, q = g % 6u;
         const BuildNode& N = B.nodes[node];
-        if (N.count > kBuildBig) continue;  // build_cov_big
+        if (N.count > B.big_min) continue;  // build_cov_big
         B.mom[9ull * (node - B.lo) + 3u + q] = chain_sum(B.Tm + q * n3 + 3ull * N.begin, 3u * N.count);
     }
 }
@@ -527,7 +538,6 @@ struct Replay {
 // triangles, and 2,048 with 64 threads (ten blocks an SM) for smaller ones.
 using ReplayBig = Replay<8192>;
 using ReplayMid = Replay<2048>;
-constexpr uint32_t kReplayMid = 1024;
 
 __device__ __forceinline__ uint32_t tile_at(uint32_t j) { return j + (j >> 4); }
 
@@ -693,13 +703,13 @@ __device__ double replay_sum(const double* __restrict__ x, uint32_t n, Replay<kT
     return s;
 }
 
-// Whether a node of more than kBuildBig triangles is this tile size's.
+// Whether a node of the list is this tile size's.
 template <class R>
 __device__ __forceinline__ bool replays(uint32_t count) {
     return (count > kReplayMid) == (R::kThreads == ReplayBig::kThreads);
 }
 
-// The same for the level's nodes of more than kBuildBig triangles, a block
+// The same for the nodes of the level's list, a block
 // per product.
 template <class R>
 __global__ void __launch_bounds__(R::kThreads) build_cov_big_kernel(const BuildParams B) {
@@ -713,6 +723,25 @@ __global__ void __launch_bounds__(R::kThreads) build_cov_big_kernel(const BuildP
         if (!replays<R>(N.count)) continue;
         const double s = replay_sum(B.Tm + q * n3 + 3ull * N.begin, 3u * N.count, sh);
         if (threadIdx.x == 0u) B.mom[9ull * (id - B.lo) + 3u + q] = s;
+        __syncthreads();
+    }
+    beside_end();
+}
+
+// The coordinate sums of the list's nodes that replays_sums names, a block per
+// node and coordinate.
+__global__ void __launch_bounds__(ReplayMid::kThreads) build_sums_mid_kernel(const BuildParams B) {
+    beside(B);
+    extern __shared__ __align__(16) unsigned char smem[];
+    ReplayMid& sh = *reinterpret_cast<ReplayMid*>(smem);
+    const uint64_t n3 = 3ull * B.T;
+    for (uint32_t i = blockIdx.x; i < 3u * B.n_big; i += gridDim.x) {
+        const uint32_t id = B.big[i / 3u], c = i % 3u;
+        const BuildNode& N = B.nodes[id];
+        if (!replays_sums(B, N.count)) continue;
+        const uint32_t np = 3u * N.count;
+        const double s = replay_sum(B.D + c * n3 + 3ull * N.begin, np, sh);
+        if (threadIdx.x == 0u) B.mom[9ull * (id - B.lo) + c] = s / double(np);
         __syncthreads();
     }
     beside_end();
@@ -1005,19 +1034,34 @@ __device__ __forceinline__ uint32_t add_children(const BuildParams& B, BuildNode
     return k;
 }
 
-constexpr uint32_t kSmall = 16;  // nodes of at most this many triangles: a thread each
+// Nodes of at most kSmall triangles: a thread each in a level of more than
+// kNarrow nodes an SM, where the boxes' FP64 instructions bound (a warp's take
+// the time of a lane's); else a warp each, as a lane's walk over 16 triangles
+// takes 40 us and a warp's 10: a 5,003-triangle mesh 2,711 to 2,547 us, 256
+// meshes of 1.4 M triangles (whose last levels are narrow) 21.9 to 21.5 ms.
+constexpr uint32_t kSmall = 16, kNarrow = 128;
 
-// A warp per node of the level with more than kSmall and at most kBuildBig
+// A warp per node of the level with more than small_max and at most big_min
 // triangles: the box, the split, the children's positions.
 __global__ void __launch_bounds__(128) build_fit_kernel(const BuildParams B) {
-    beside(B);
+    if (B.small_max)  // after build_fit_small's start
+        beside(B);
+    else
+        after_all(B);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t id = B.lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); id < B.hi; id += warps) {
         BuildNode& N = B.nodes[id];
         const uint32_t begin = N.begin, n = N.count;
-        if (n <= kSmall || n > kBuildBig) continue;
+        if ((B.small_max && n <= B.small_max) || n > B.big_min) continue;
         const Box box = fit_warp(B, begin, n, B.mom + 9ull * (id - B.lo), lane);
+        if (n <= kLeafMax) {
+            if (lane == 0u) {
+                store_box(N, box);
+                N.kid = kNoKid;
+            }
+            continue;
+        }
         const uint32_t nl = split_node(B.Pp + 9ull * begin, B.perm + begin, B.scratch + begin, n, box, lane);
         uint32_t k = 0;
         if (lane == 0u) {
@@ -1038,13 +1082,13 @@ __device__ __forceinline__ void merge_ext(Ext& e, const Ext& o, bool lo) {
     if ((lo ? o.k < e.k : o.k > e.k) || (o.k == e.k && o.j > e.j)) e = o;
 }
 
-// A block per node of the level's list of nodes of more than kBuildBig
+// A block per node of the level's list of nodes of more than big_min
 // triangles (the top levels of the large meshes, where one warp's walk of the
 // range set the level's time): the box and split of build_fit_kernel, the
 // corners shared out by thread, the split's counts and partition by warp over
 // consecutive segments of the range (each warp's lefts and rights go after
 // those of the segments before it, so the partition stays stable). Children
-// of more than kBuildBig triangles go to the next level's list.
+// of more than big_min triangles go to the next level's list.
 __global__ void __launch_bounds__(kBigWarps * 32) build_fit_big_kernel(const BuildParams B) {
     beside(B);
     constexpr uint32_t NT = kBigWarps * 32u;
@@ -1172,8 +1216,8 @@ __global__ void __launch_bounds__(kBigWarps * 32) build_fit_big_kernel(const Bui
             N.kid = kNoKid;
             const uint32_t k = add_children(B, N, nl);
             if (k != kNoKid) {
-                if (nl > kBuildBig) B.big_out[atomicAdd(B.n_big_out, 1u)] = k;
-                if (n - nl > kBuildBig) B.big_out[atomicAdd(B.n_big_out, 1u)] = k + 1u;
+                if (nl > B.big_min) B.big_out[atomicAdd(B.n_big_out, 1u)] = k;
+                if (n - nl > B.big_min) B.big_out[atomicAdd(B.n_big_out, 1u)] = k + 1u;
             }
             s_kid = k;
         }
@@ -1186,13 +1230,13 @@ __global__ void __launch_bounds__(kBigWarps * 32) build_fit_big_kernel(const Bui
     beside_end();
 }
 
-// A thread per node of the level with at most kSmall triangles.
+// A thread per node of the level with at most small_max triangles.
 __global__ void __launch_bounds__(128) build_fit_small_kernel(const BuildParams B) {
     after_all(B);
     for (uint32_t id = B.lo + blockIdx.x * blockDim.x + threadIdx.x; id < B.hi; id += gridDim.x * blockDim.x) {
         BuildNode& N = B.nodes[id];
         const uint32_t begin = N.begin, n = N.count;
-        if (n > kSmall) continue;
+        if (n > B.small_max) continue;
         const Box box = fit_thread(B, begin, n, B.mom + 9ull * (id - B.lo));
         store_box(N, box);
         N.kid = kNoKid;
@@ -1435,6 +1479,8 @@ cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStre
     run(build_sums_kernel, g_sum, 128, 0, p.n_big ? 1u : g_tri);
     if (p.n_big) {
         const uint32_t g_due = grid(3ull * p.n_big);
+        const bool few = p.big_min == kBuildBigFew;
+        if (few) run(build_sums_mid_kernel, blocks(3ull * p.n_big), ReplayMid::kThreads, sizeof(ReplayMid), 1u);
         run(build_sums_big_kernel, blocks(p.n_big), kBigWarps * 32u, 0, g_due);
         run(build_sums_due_kernel, g_due, 128, 0, g_tri);
     }
@@ -1447,9 +1493,14 @@ cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStre
     }
     run(build_eig_kernel, g_node, 128, 0, g_tri);
     run(build_proj_kernel, g_tri, 128, 0, g_node);
-    run(build_fit_small_kernel, g_node, 128, 0, 1u);
+    q.small_max = width <= kNarrow * sm_count ? 0u : kSmall;
+    const uint32_t g_warp = blocks((width + 3u) / 4u);
+    if (q.small_max)
+        run(build_fit_small_kernel, g_node, 128, 0, 1u);
+    else
+        run(build_fit_kernel, g_warp, 128, 0, 1u);
     if (p.n_big) run(build_fit_big_kernel, blocks(p.n_big), kBigWarps * 32u, 0, 1u);
-    run(build_fit_kernel, blocks((width + 3u) / 4u), 128, 0, ~0u);
+    if (q.small_max) run(build_fit_kernel, g_warp, 128, 0, ~0u);
     return e;
 }
 

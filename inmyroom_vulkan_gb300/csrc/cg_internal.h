@@ -499,13 +499,24 @@ struct BuildParams {
     uint32_t* node_ctr;      // [0] next free node, [1] error, [2 + parity] nodes in big_out
     uint32_t node_cap;
     unsigned* error;
-    const uint32_t* big;     // this level's nodes of more than kBuildBig triangles (a block fits each)
+    const uint32_t* big;     // this level's nodes of more than big_min triangles
     uint32_t n_big;
     uint32_t* big_out;       // the next level's, appended by the splits of this level's
     uint32_t* n_big_out;
+    uint32_t big_min;        // nodes of more triangles than this are in `big`, a block (or several) each
+    uint32_t small_max;      // nodes of at most this many triangles are fitted by a thread each
     bool early;              // the next kernel's blocks may start beside this one
 };
-constexpr uint32_t kBuildBig = 256;  // nodes of more than this many triangles are fitted by a block
+// The nodes that blocks handle (big_min): of more than 256 triangles; of more
+// than 128 in a batch of few triangles (at most 256 an SM). A chain of 3 x 256
+// terms takes 26 us or more, segments of it by a block 15, but for six times
+// the FP64 instructions, which only a batch of few triangles leaves room for:
+// a 5,003-triangle mesh 2,640 to 2,547 us, eight meshes of 20,000 triangles
+// together 2,877 to 2,804, but 16 of 62,000 would take 4,600 instead of 4,355.
+constexpr uint32_t kBuildBig = 256, kBuildBigFew = 128, kBuildFew = 256;
+inline uint32_t build_big_min(uint64_t triangles, uint32_t sm_count) {
+    return triangles <= uint64_t(kBuildFew) * sm_count ? kBuildBigFew : kBuildBig;
+}
 cudaError_t build_smem_limit();
 cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStream_t s);
 struct BuildMesh {

@@ -10,7 +10,7 @@ from test_gpu_build import M, same
 
 pytestmark = pytest.mark.gpu
 
-EDGES = [4, 5, 16, 17, 33, 256, 257, 513, 682, 683, 1024, 1025, 2730, 2731, 5462]
+EDGES = [4, 5, 16, 17, 33, 128, 129, 256, 257, 513, 682, 683, 1024, 1025, 2730, 2731, 5462]
 
 
 def mesh(n, seed):
@@ -19,7 +19,7 @@ def mesh(n, seed):
     return M(pts, rng.integers(0, len(pts), (n, 3)))
 
 
-@pytest.mark.parametrize("sizes", [[n] for n in EDGES] + [EDGES, EDGES[::-1]], ids=lambda s: "-".join(map(str, s)))
+@pytest.mark.parametrize("sizes", [[n] for n in EDGES] + [EDGES, EDGES * 3], ids=lambda s: f"{len(s)}x{s[0]}")
 def test_sizes(gpu_ctx, port, sizes):
     meshes = [mesh(n, 100 + n) for n in sizes]
     ids = gpu_ctx.build_trees(meshes)
