@@ -20,8 +20,9 @@
 //   build_cov     a thread per node and product: the covariance sum in
 //                 corner order (build_cov_big: a block per product of a node
 //                 of more than big_min triangles)
-//   build_eig     a thread per node: eig3 of the covariance in FP64; the
-//                 box axes are the rows of the eigenvector matrix
+//   build_eig     a thread per node (build_eig_group: a group of lanes in a
+//                 narrow level): eig3 of the covariance in FP64; the box axes
+//                 are the rows of the eigenvector matrix
 //   build_proj    a thread per triangle position: its corners' FP64
 //                 projections on its node's axes
 //   build_fit     a warp per node (build_fit_small: a thread per node of at
@@ -759,12 +760,46 @@ __global__ void build_eig_kernel(const BuildParams B) {
         const double cxx = m[3], cyy = m[4], czz = m[5], cxy = m[6], cxz = m[7], cyz = m[8];
         double v[3][3] = {{cxx / dn, cxy / dn, cxz / dn}, {cxy / dn, cyy / dn, cyz / dn}, {cxz / dn, cyz / dn, czz / dn}};
         double d[3], off[3];
-        tridiagonalize(v, d, off);
-        ql_sort(v, d, off, 2.220446049250313e-16);  // 2^-52
+        tridiagonalize(Alone{}, v, d, off);
+        ql_sort(Alone{}, v, d, off, 2.220446049250313e-16);  // 2^-52
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
             for (int c = 0; c < 3; ++c) m[3 * r + c] = v[r][c];
+    }
+}
+
+// The same by `lanes` lanes a node (4, 8, 16 or 32): a narrow level's time is
+// that of one node's chain of FP64 instructions, 74 cycles each for a lane as
+// for a warp. The group's lanes share the quotients and the rows out, and with
+// fewer nodes in a warp fewer wait for another's sweeps: all levels of a
+// 5,003-triangle mesh 644 to 540 us (its build 2,515 to 2,415), the build of
+// eight meshes of up to 5,000 triangles 2,800 to 2,685. The widest groups that
+// leave a warp a scheduler; and the blocks do not start early, as two of them
+// on one SM then take twice the time (the eight meshes 2,860).
+__global__ void build_eig_group_kernel(const BuildParams B, uint32_t lanes) {
+    after_all(B);
+    const uint32_t lane = threadIdx.x & 31u, base = lane & ~(lanes - 1u), k = (lane - base) & 3u;
+    const unsigned mask = lanes == 32u ? kAll : ((1u << lanes) - 1u) << base;
+    const Group by{mask, base, (k & 1u) != 0u};
+    for (uint32_t node = B.lo + (blockIdx.x * blockDim.x + threadIdx.x) / lanes; node < B.hi;
+         node += gridDim.x * blockDim.x / lanes) {
+        double* m = B.mom + 9ull * (node - B.lo);
+        if (B.nodes[node].count == 0u) continue;
+        const double dn = double(3u * B.nodes[node].count);
+        double c[6];  // xx, yy, zz, xy, xz, yz
+#pragma unroll
+        for (int i = 0; i < 6; i += 2) by.divide(m[3 + i], m[4 + i], dn, c[i], c[i + 1]);
+        double v[3][3] = {{c[0], c[3], c[4]}, {c[3], c[1], c[5]}, {c[4], c[5], c[2]}};
+        double d[3], off[3];
+        tridiagonalize(by, v, d, off);
+        double w[1][3];  // row k (k = 3: row 2 again)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) w[0][i] = k == 0u ? v[0][i] : k == 1u ? v[1][i] : v[2][i];
+        ql_sort(by, w, d, off, 2.220446049250313e-16);  // 2^-52
+        if (lane - base < 3u)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) m[3u * k + i] = w[0][i];
     }
 }
 
@@ -1485,13 +1520,22 @@ cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStre
         run(build_sums_due_kernel, g_due, 128, 0, g_tri);
     }
     run(build_terms_kernel, g_tri, 128, 0, g_cov);
-    run(build_cov_kernel, g_cov, 128, 0, p.n_big ? 1u : g_node);
+    uint32_t lanes = width <= 32u * sm_count ? 32u : 0u;  // of a node's eigensystem, where that is four or more
+    while (uint64_t(width) * lanes > 128u * sm_count) lanes >>= 1;
+    const uint32_t g_eig = grid(uint64_t(width) * (lanes ? lanes : 1u));
+    const uint32_t g_even = lanes ? ~0u : g_eig;  // never early
+    run(build_cov_kernel, g_cov, 128, 0, p.n_big ? 1u : g_even);
     if (p.n_big) {
         const uint32_t g = blocks(6ull * p.n_big);
         run(build_cov_big_kernel<ReplayBig>, g, ReplayBig::kThreads, sizeof(ReplayBig), 1u);
-        run(build_cov_big_kernel<ReplayMid>, g, ReplayMid::kThreads, sizeof(ReplayMid), g_node);
+        run(build_cov_big_kernel<ReplayMid>, g, ReplayMid::kThreads, sizeof(ReplayMid), g_even);
     }
-    run(build_eig_kernel, g_node, 128, 0, g_tri);
+    if (lanes) {
+        q.early = g_tri <= sm_count;
+        if (e == cudaSuccess) e = next(build_eig_group_kernel, g_eig, 128, 0, s, q, lanes);
+    } else {
+        run(build_eig_kernel, g_node, 128, 0, g_tri);
+    }
     run(build_proj_kernel, g_tri, 128, 0, g_node);
     q.small_max = width <= kNarrow * sm_count ? 0u : kSmall;
     const uint32_t g_warp = blocks((width + 3u) / 4u);

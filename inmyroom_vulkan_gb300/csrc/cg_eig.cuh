@@ -22,11 +22,37 @@ __device__ __forceinline__ R hyp(R x, R y) {
 // 5,003-triangle mesh's build 724 us instead of 644 (there FP64 instructions,
 // about 64 cycles each, are the rest).
 
+// How a matrix is worked on: by one thread (Alone), or by a group of lanes that
+// all hold it (Group: 4 to 32 lanes of a warp, of which mask are this group's
+// and base the first), where two quotients of one divisor take the time of one
+// division, a lane each. kRows rows of v to a thread: a Group's lane turns one
+// row in the QL sweeps.
+struct Alone {
+    static constexpr int kRows = 3;
+    template <typename R>
+    __device__ __forceinline__ void divide(R a, R b, R by, R& qa, R& qb) const {
+        qa = a / by;
+        qb = b / by;
+    }
+};
+struct Group {
+    static constexpr int kRows = 1;
+    unsigned mask;
+    uint32_t base;
+    bool odd;  // this lane's is the second quotient
+    template <typename R>
+    __device__ __forceinline__ void divide(R a, R b, R by, R& qa, R& qb) const {
+        const R q = (odd ? b : a) / by;
+        qa = __shfl_sync(mask, q, base);
+        qb = __shfl_sync(mask, q, base + 1u);
+    }
+};
+
 // Householder reduction of the symmetric 3x3 in v to tridiagonal form
 // (eig3.cpp:21-134): v becomes the accumulated transform, d the diagonal,
 // e[1..2] the sub-diagonal.
-template <typename R>
-__device__ __forceinline__ void tridiagonalize(R v[3][3], R d[3], R e[3]) {
+template <class By, typename R>
+__device__ __forceinline__ void tridiagonalize(const By& by, R v[3][3], R d[3], R e[3]) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) d[c] = v[2][c];
 #pragma unroll
@@ -43,11 +69,12 @@ __device__ __forceinline__ void tridiagonalize(R v[3][3], R d[3], R e[3]) {
                 v[c][i] = R(0);
             }
         } else {
+            if (i == 2)
+                by.divide(d[0], d[1], scale, d[0], d[1]);
+            else
+                d[0] = d[0] / scale;
 #pragma unroll
-            for (int k = 0; k < i; ++k) {
-                d[k] = d[k] / scale;
-                h = h + d[k] * d[k];
-            }
+            for (int k = 0; k < i; ++k) h = h + d[k] * d[k];
             R f = d[i - 1];
             R g = sqrt(h);
             if (f > 0) g = -g;
@@ -69,11 +96,12 @@ __device__ __forceinline__ void tridiagonalize(R v[3][3], R d[3], R e[3]) {
                 e[c] = g;
             }
             f = R(0);
+            if (i == 2)
+                by.divide(e[0], e[1], h, e[0], e[1]);
+            else
+                e[0] = e[0] / h;
 #pragma unroll
-            for (int c = 0; c < i; ++c) {
-                e[c] = e[c] / h;
-                f = f + e[c] * d[c];
-            }
+            for (int c = 0; c < i; ++c) f = f + e[c] * d[c];
             const R hh = f / (h + h);
 #pragma unroll
             for (int c = 0; c < i; ++c) e[c] = e[c] - hh * d[c];
@@ -95,8 +123,10 @@ __device__ __forceinline__ void tridiagonalize(R v[3][3], R d[3], R e[3]) {
         v[i][i] = R(1);
         const R h = d[i + 1];
         if (h != R(0)) {
-#pragma unroll
-            for (int k = 0; k <= i; ++k) d[k] = v[k][i + 1] / h;
+            if (i == 1)
+                by.divide(v[0][2], v[1][2], h, d[0], d[1]);
+            else
+                d[0] = v[0][1] / h;
 #pragma unroll
             for (int c = 0; c <= i; ++c) {
                 R g = R(0);
@@ -121,8 +151,8 @@ __device__ __forceinline__ void tridiagonalize(R v[3][3], R d[3], R e[3]) {
 // Sweeps of the implicit-shift QL over rows L..M (eig3.cpp:160-227) until
 // e[L] is negligible. A sweep count limit stops what only a non-finite input
 // could run forever.
-template <int L, int M, typename R>
-__device__ __forceinline__ void ql_sweeps(R v[3][3], R d[3], R e[3], R& f, R small) {
+template <int L, int M, class By, typename R>
+__device__ __forceinline__ void ql_sweeps(const By& by, R v[By::kRows][3], R d[3], R e[3], R& f, R small) {
     int sweeps = 0;
     do {
         ++sweeps;
@@ -150,12 +180,11 @@ __device__ __forceinline__ void ql_sweeps(R v[3][3], R d[3], R e[3], R& f, R sma
             h = c * p;
             r = hyp(p, e[i]);
             e[i + 1] = s * r;
-            s = e[i] / r;
-            c = p / r;
+            by.divide(e[i], p, r, s, c);
             p = c * d[i] - s * g;
             d[i + 1] = h + s * (c * g + s * d[i]);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < By::kRows; ++k) {
                 h = v[k][i + 1];
                 v[k][i + 1] = s * v[k][i] + c * h;
                 v[k][i] = c * v[k][i] - s * h;
@@ -168,10 +197,11 @@ __device__ __forceinline__ void ql_sweeps(R v[3][3], R d[3], R e[3], R& f, R sma
 }
 
 // Implicit-shift QL on the tridiagonal form, then the ascending sort of the
-// eigenvalues with their eigenvector columns (eig3.cpp:138-254). The last row
+// eigenvalues with their eigenvector columns (eig3.cpp:138-254), for the rows of
+// v that the thread has. The last row
 // with a negligible sub-diagonal is at most 2 (its e is 0).
-template <typename R>
-__device__ __forceinline__ void ql_sort(R v[3][3], R d[3], R e[3], R eps) {
+template <class By, typename R>
+__device__ __forceinline__ void ql_sort(const By& by, R v[By::kRows][3], R d[3], R e[3], R eps) {
     e[0] = e[1], e[1] = e[2];
     e[2] = R(0);
     R f = 0, tst1 = 0;
@@ -182,14 +212,14 @@ __device__ __forceinline__ void ql_sort(R v[3][3], R d[3], R e[3], R eps) {
     top(0);
     if (!(fabs(e[0]) <= eps * tst1)) {
         if (fabs(e[1]) <= eps * tst1)
-            ql_sweeps<0, 1>(v, d, e, f, eps * tst1);
+            ql_sweeps<0, 1>(by, v, d, e, f, eps * tst1);
         else
-            ql_sweeps<0, 2>(v, d, e, f, eps * tst1);
+            ql_sweeps<0, 2>(by, v, d, e, f, eps * tst1);
     }
     d[0] = d[0] + f;
     e[0] = R(0);
     top(1);
-    if (!(fabs(e[1]) <= eps * tst1)) ql_sweeps<1, 2>(v, d, e, f, eps * tst1);
+    if (!(fabs(e[1]) <= eps * tst1)) ql_sweeps<1, 2>(by, v, d, e, f, eps * tst1);
     d[1] = d[1] + f;
     e[1] = R(0);
     d[2] = d[2] + f;
@@ -209,7 +239,7 @@ __device__ __forceinline__ void ql_sort(R v[3][3], R d[3], R e[3], R eps) {
                 d[j] = d[i];
                 d[i] = p;
 #pragma unroll
-                for (int r = 0; r < 3; ++r) {
+                for (int r = 0; r < By::kRows; ++r) {
                     const R tmp = v[r][i];
                     v[r][i] = v[r][j];
                     v[r][j] = tmp;

@@ -222,8 +222,8 @@ __global__ void refit_axes_kernel(const RefitTree* trees, const RefitBufs B) {
     for (int i = 0; i < 6; ++i) c[i] = m.m2[i] / fn;  // xx, yy, zz, xy, xz, yz
     float v[3][3] = {{c[0], c[3], c[4]}, {c[3], c[1], c[5]}, {c[4], c[5], c[2]}};
     float d[3], e[3];
-    tridiagonalize(v, d, e);
-    ql_sort(v, d, e, FLT_EPSILON);
+    tridiagonalize(Alone{}, v, d, e);
+    ql_sort(Alone{}, v, d, e, FLT_EPSILON);
     ax[0] = make_float4(v[0][0], v[0][1], v[0][2], 1.f);
     ax[1] = make_float4(v[1][0], v[1][1], v[1][2], 0.f);
     ax[2] = make_float4(v[2][0], v[2][1], v[2][2], 0.f);

@@ -29,6 +29,18 @@ def test_sizes(gpu_ctx, port, sizes):
         gpu_ctx.free_tree(int(tid))
 
 
+@pytest.mark.parametrize("n", [152, 153, 609, 4864, 4865])
+def test_level_widths(gpu_ctx, port, n):
+    """Levels of n nodes, where the eigensystems' group of lanes changes."""
+    kinds = [mesh(k, 31 + k) for k in (1, 5, 7, 12)]
+    ids = gpu_ctx.build_trees([kinds[i % 4] for i in range(n)])
+    for i in list(range(8)) + list(range(n - 8, n)):
+        m = kinds[i % 4]
+        same(gpu_ctx.export_tree(int(ids[i])), port.tree_build(m.points, m.indices, None).export(), normals=False)
+    for tid in ids:
+        gpu_ctx.free_tree(int(tid))
+
+
 def test_wide_level(gpu_ctx, port):
     """20,000 small meshes beside large ones: every per-node grid is above a block an SM."""
     small = [mesh(n, 7 + n) for n in (1, 5, 6, 9, 17, 20)]
