@@ -11,20 +11,18 @@
 // reference (std::accumulate, std::inner_product), so each is one thread's
 // chain here; the FP64 pipe of this part is narrow, so everything around the
 // chains runs a thread per corner on every SM:
-//   build_points  a thread per triangle position: its corners as doubles
+//   build_points  a thread per corner: as doubles
 //   build_sums    a thread per node and coordinate: the sum in corner order,
 //                 the mean (build_sums_mid, build_sums_big: blocks for a
 //                 node of more than big_min triangles)
-//   build_terms   a thread per triangle position: the six centred products
-//                 of its corners
+//   build_terms   a thread per corner: its six centred products
 //   build_cov     a thread per node and product: the covariance sum in
 //                 corner order (build_cov_big: a block per product of a node
 //                 of more than big_min triangles)
 //   build_eig     a thread per node (build_eig_group: a group of lanes in a
 //                 narrow level): eig3 of the covariance in FP64; the box axes
 //                 are the rows of the eigenvector matrix
-//   build_proj    a thread per triangle position: its corners' FP64
-//                 projections on its node's axes
+//   build_proj    a thread per corner: its FP64 projections on its node's axes
 //   build_fit     a warp per node (build_fit_small: a thread per node of at
 //                 most 16 triangles of a wide level; build_fit_big: a block
 //                 per node of more than big_min): fewer than two distinct
@@ -146,23 +144,26 @@ __device__ __forceinline__ void beside_end() {
 
 // The corners of the level's triangles at their triangle's position: as
 // doubles by coordinate, and as floats by position (so that a node reads its
-// corners contiguously); a thread per position (positions of earlier levels'
-// leaves are skipped).
+// corners contiguously); a thread per corner (positions of earlier levels'
+// leaves are skipped). This kernel and the two below it that fill arrays by
+// corner store whole sectors so; with a thread per triangle, its corners'
+// stores 24 bytes apart, a level of 1.4 M triangles took 100 us instead of 47
+// for the corners and 104 instead of 76 for the products (of FP64 instructions
+// alone 65; the projections' 115 are all theirs).
 __global__ void build_points_kernel(const BuildParams B) {
     after_all(B);
-    const uint64_t n3 = 3ull * B.T;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < B.T; t += gridDim.x * blockDim.x) {
-        const uint32_t o = B.own[t];
+    const uint32_t n3 = 3u * B.T;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n3; j += gridDim.x * blockDim.x) {
+        const uint32_t t = j / 3u, o = B.own[t];
         if (o < B.lo || o >= B.hi) continue;
-        const float* q = B.P + 9ull * B.perm[t];
-        float* pp = B.Pp + 9ull * t;
+        const float* q = B.P + 9ull * B.perm[t] + 3u * (j - 3u * t);
+        float* pp = B.Pp + 3ull * j;
+        const float x[3] = {q[0], q[1], q[2]};
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                B.D[c * n3 + 3ull * t + k] = double(q[3 * k + c]);
-                pp[3 * k + c] = q[3 * k + c];
-            }
+        for (int c = 0; c < 3; ++c) {
+            B.D[uint64_t(c) * n3 + j] = double(x[c]);
+            pp[c] = x[c];
+        }
     }
 }
 
@@ -463,27 +464,22 @@ __global__ void build_sums_due_kernel(const BuildParams B) {
     }
 }
 
-// The centred products of every corner of the level, a thread per position:
+// The centred products of every corner of the level, a thread per corner:
 // xx, yy, zz, xy, xz, yz (OBB.cpp:57-74).
 __global__ void build_terms_kernel(const BuildParams B) {
     after_all(B);
     const uint64_t n3 = 3ull * B.T;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < B.T; t += gridDim.x * blockDim.x) {
-        const uint32_t o = B.own[t];
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n3; j += gridDim.x * blockDim.x) {
+        const uint32_t o = B.own[j / 3u];
         if (o < B.lo || o >= B.hi) continue;
         const double* m = B.mom + 9ull * (o - B.lo);
-        const double mx = m[0], my = m[1], mz = m[2];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const uint64_t j = 3ull * t + k;
-            const double dx = B.D[j] - mx, dy = B.D[n3 + j] - my, dz = B.D[2 * n3 + j] - mz;
-            B.Tm[j] = dx * dx;
-            B.Tm[n3 + j] = dy * dy;
-            B.Tm[2 * n3 + j] = dz * dz;
-            B.Tm[3 * n3 + j] = dx * dy;
-            B.Tm[4 * n3 + j] = dx * dz;
-            B.Tm[5 * n3 + j] = dy * dz;
-        }
+        const double dx = B.D[j] - m[0], dy = B.D[n3 + j] - m[1], dz = B.D[2 * n3 + j] - m[2];
+        B.Tm[j] = dx * dx;
+        B.Tm[n3 + j] = dy * dy;
+        B.Tm[2 * n3 + j] = dz * dz;
+        B.Tm[3 * n3 + j] = dx * dy;
+        B.Tm[4 * n3 + j] = dx * dz;
+        B.Tm[5 * n3 + j] = dy * dz;
     }
 }
 
@@ -804,30 +800,25 @@ __global__ void build_eig_group_kernel(const BuildParams B, uint32_t lanes) {
 }
 
 // The projections of every corner of the level on its node's three axes
-// (the dot products of OBB.cpp:117, 136, 155), a thread per triangle
-// position, into the products' buffer (free once the covariances are
-// summed): [axis][corner].
+// (the dot products of OBB.cpp:117, 136, 155), a thread per corner, into the
+// products' buffer (free once the covariances are summed): [axis][corner].
 __global__ void build_proj_kernel(const BuildParams B) {
     after_all(B);
     const uint64_t n3 = 3ull * B.T;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < B.T; t += gridDim.x * blockDim.x) {
-        const uint32_t o = B.own[t];
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n3; j += gridDim.x * blockDim.x) {
+        const uint32_t o = B.own[j / 3u];
         if (o < B.lo || o >= B.hi) continue;
         const double* ax = B.mom + 9ull * (o - B.lo);
         double a[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) a[k] = ax[k];
+        const double px = B.D[j], py = B.D[n3 + j], pz = B.D[2 * n3 + j];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const uint64_t j = 3ull * t + k;
-            const double px = B.D[j], py = B.D[n3 + j], pz = B.D[2 * n3 + j];
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                double pr = a[3 * r] * px;
-                pr = pr + a[3 * r + 1] * py;
-                pr = pr + a[3 * r + 2] * pz;
-                B.Tm[r * n3 + j] = pr;
-            }
+        for (int r = 0; r < 3; ++r) {
+            double pr = a[3 * r] * px;
+            pr = pr + a[3 * r + 1] * py;
+            pr = pr + a[3 * r + 2] * pz;
+            B.Tm[r * n3 + j] = pr;
         }
     }
 }
@@ -1494,13 +1485,12 @@ cudaError_t next(void (*kernel)(P...), uint32_t blocks, uint32_t threads, size_t
 cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStream_t s) {
     if (p.hi <= p.lo) return cudaSuccess;
     const uint32_t width = p.hi - p.lo;
-    const uint32_t wide = sm_count * 8u;  // blocks of the per-position kernels
-    auto grid = [&](uint64_t threads) {
-        const uint64_t b = (threads + 127u) / 128u;
+    auto grid = [&](uint64_t threads, uint32_t per_sm = 8u) {
+        const uint64_t b = (threads + 127u) / 128u, wide = uint64_t(sm_count) * per_sm;
         return uint32_t(b < wide ? (b ? b : 1u) : wide);
     };
     auto blocks = [](uint64_t b) { return uint32_t(b < 65535u ? b : 65535u); };
-    const uint32_t g_tri = grid(p.T), g_sum = grid(3ull * width), g_cov = grid(6ull * width), g_node = grid(width);
+    const uint32_t g_tri = grid(3ull * p.T, 16u), g_sum = grid(3ull * width), g_cov = grid(6ull * width), g_node = grid(width);
     BuildParams q = p;
     q.early = g_sum <= sm_count;
     build_points_kernel<<<g_tri, 128, 0, s>>>(q);
