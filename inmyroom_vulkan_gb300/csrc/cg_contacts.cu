@@ -253,16 +253,40 @@ __device__ __forceinline__ uint32_t n_slots(const ContactParams& P) {
     return n < P.table_mask + 1u ? n : P.table_mask + 1u;
 }
 
+// The threads that work on a map together: a whole block, or half of one (its
+// threads wait at a barrier of their own).
+template <uint32_t T>
+struct Team {
+    uint32_t t;    // this thread's place
+    uint32_t bar;  // barrier: 0, the block's; 1 and 2, its halves'
+    __device__ __forceinline__ static constexpr uint32_t size() { return T; }
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory"); }
+    __device__ __forceinline__ bool any(bool x) const {
+        uint32_t r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(r)
+            : "r"(uint32_t(x)), "r"(bar), "n"(T)
+            : "memory");
+        return r != 0u;
+    }
+};
+struct Block {  // of any size
+    uint32_t t = threadIdx.x;
+    __device__ __forceinline__ static uint32_t size() { return blockDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+
 // Exclusive scans by one block (blockDim.x a multiple of 32, at most 1024) of
 // get1(0..n1-1) and get2(0..n2-1) side by side: each thread takes a
 // contiguous run of each, the runs' sums are scanned with warp shuffles, every
 // warp adds up the partial sums of the warps before it, put(i, prefix) is
 // called in order within each run. Two barriers; the totals go to every
 // thread. `part` holds 64 words. get must return the same value twice.
-template <class Get1, class Put1, class Get2, class Put2>
-__device__ void block_scan2(uint32_t n1, uint32_t n2, uint32_t* part, Get1 get1, Put1 put1, Get2 get2, Put2 put2,
+template <class Tm, class Get1, class Put1, class Get2, class Put2>
+__device__ void block_scan2(const Tm& team, uint32_t n1, uint32_t n2, uint32_t* part, Get1 get1, Put1 put1, Get2 get2, Put2 put2,
                             uint32_t& total1, uint32_t& total2) {
-    const uint32_t T = blockDim.x, t = threadIdx.x, lane = t & 31u, warp = t >> 5, nw = T >> 5;
+    const uint32_t T = team.size(), t = team.t, lane = t & 31u, warp = t >> 5, nw = T >> 5;
     const uint32_t per1 = (n1 + T - 1u) / T, a0 = min(n1, t * per1), a1 = min(n1, a0 + per1);
     const uint32_t per2 = (n2 + T - 1u) / T, c0 = min(n2, t * per2), c1 = min(n2, c0 + per2);
     uint32_t s1 = 0, s2 = 0;
@@ -282,7 +306,7 @@ __device__ void block_scan2(uint32_t n1, uint32_t n2, uint32_t* part, Get1 get1,
         part[warp] = i1;
         part[32u + warp] = i2;
     }
-    __syncthreads();
+    team.sync();
     uint32_t b1 = 0, b2 = 0, t1 = 0, t2 = 0;
     for (uint32_t w = 0; w < nw; ++w) {
         const uint32_t p1 = part[w], p2 = part[32u + w];
@@ -304,18 +328,18 @@ __device__ void block_scan2(uint32_t n1, uint32_t n2, uint32_t* part, Get1 get1,
         put2(i, r2);
         r2 += v;
     }
-    __syncthreads();
+    team.sync();
     total1 = t1;
     total2 = t2;
 }
 
 // One exclusive scan of get(0..n-1) (block_scan2 with an empty second).
 // Returns the total.
-template <class Get, class Put>
-__device__ uint32_t block_scan(uint32_t n, uint32_t* part, Get get, Put put) {
+template <class Tm, class Get, class Put>
+__device__ uint32_t block_scan(const Tm& team, uint32_t n, uint32_t* part, Get get, Put put) {
     uint32_t total = 0, none = 0;
     block_scan2(
-        n, 0u, part, get, put, [](uint32_t) { return 0u; }, [](uint32_t, uint32_t) {}, total, none);
+        team, n, 0u, part, get, put, [](uint32_t) { return 0u; }, [](uint32_t, uint32_t) {}, total, none);
     return total;
 }
 
@@ -480,11 +504,11 @@ __device__ void paired_path(const PackedQuery* queries, const DevTree* trees, co
 }
 
 // Ascending bitonic sort of n2 (a power of two) entries by the whole block.
-template <class K, class Less>
-__device__ void bitonic(K* a, uint32_t n2, Less less) {
+template <class Tm, class K, class Less>
+__device__ void bitonic(const Tm& team, K* a, uint32_t n2, Less less) {
     for (uint32_t k = 2; k <= n2; k <<= 1)
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) {
+            for (uint32_t i = team.t; i < n2; i += team.size()) {
                 const uint32_t l = i ^ j;
                 if (l > i) {
                     const K x = a[i], y = a[l];
@@ -495,7 +519,7 @@ __device__ void bitonic(K* a, uint32_t n2, Less less) {
                     }
                 }
             }
-            __syncthreads();
+            team.sync();
         }
 }
 
@@ -567,8 +591,8 @@ __device__ __forceinline__ void k_keep(K& x, const K& y, bool keep_min) {
 // within a warp by shuffles, across warps through xchg (n2 keys of shared
 // memory, two barriers), between a thread's own keys in registers.
 template <uint32_t T, class K, int E>
-__device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg) {
-    const uint32_t t = threadIdx.x;
+__device__ __forceinline__ void block_sort_regs(const Team<T>& team, K (&x)[E], uint32_t n2, K* xchg) {
+    const uint32_t t = team.t;
     const bool active = t < n2;  // warp-uniform: n2 is a multiple of 32
     for (uint32_t k = 2; k <= n2; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -592,7 +616,7 @@ __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg)
 #pragma unroll
                     for (int e = 0; e < E; ++e) xchg[t + T * e] = x[e];
                 }
-                __syncthreads();
+                team.sync();
                 if (active) {
 #pragma unroll
                     for (int e = 0; e < E; ++e) {
@@ -600,7 +624,7 @@ __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg)
                         k_keep(x[e], xchg[i ^ j], ((i & j) == 0u) == ((i & k) == 0u));
                     }
                 }
-                __syncthreads();
+                team.sync();
             } else if (active) {
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
@@ -616,16 +640,16 @@ __device__ __forceinline__ void block_sort_regs(K (&x)[E], uint32_t n2, K* xchg)
 // n2 <= E * T): keys from the elements' paths and triangles,
 // sorted, then per insertion index its triangle and element.
 template <uint32_t T, class K, int E>
-__device__ __forceinline__ void insertion_order(const ContactElem* El, uint32_t n, uint32_t n2, void* xchg,
+__device__ __forceinline__ void insertion_order(const Team<T>& team, const ContactElem* El, uint32_t n, uint32_t n2, void* xchg,
                                                 uint32_t* ins_tri, uint32_t* ins_elem) {
-    const uint32_t t = threadIdx.x;
+    const uint32_t t = team.t;
     K x[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const uint32_t i = t + T * e;
         x[e] = i < n ? K::make(El[i].key_hi, El[i].key_lo, El[i].tri, i) : K::pad();
     }
-    block_sort_regs<T, K, E>(x, n2, reinterpret_cast<K*>(xchg));
+    block_sort_regs<T, K, E>(team, x, n2, reinterpret_cast<K*>(xchg));
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const uint32_t i = t + T * e;
@@ -755,7 +779,7 @@ __global__ void __launch_bounds__(256) contacts_alloc_kernel(const ContactParams
     }
     if (blockIdx.x == 0)
         block_scan(
-            2u * P.n_queries, part, [&](uint32_t i) { return P.map_cnt[i]; },
+            Block{}, 2u * P.n_queries, part, [&](uint32_t i) { return P.map_cnt[i]; },
             [&](uint32_t i, uint32_t v) { P.map_off[i] = v; });
 }
 
@@ -1056,6 +1080,7 @@ __device__ void rank_maps(const ContactParams& P) {
             start[c] = off;
             off += count[c];
             if (1u << (c > 0 ? c - 1 : 0) == kBigMap) P.ctr->n_bigmaps = off;
+            if (1u << (c > 0 ? c - 1 : 0) == kHalfMap) P.ctr->n_wholemaps = off;
         }
     }
     __syncthreads();
@@ -1069,9 +1094,9 @@ __device__ void rank_maps(const ContactParams& P) {
 __device__ void place_maps(const ContactParams& P, uint32_t* part) {
     const uint32_t m = 2u * P.n_queries;
     const uint32_t nc = block_scan(
-        m, part, [&](uint32_t i) { return P.map_fill[i]; }, [&](uint32_t i, uint32_t v) { P.map_coff[i] = v; });
+        Block{}, m, part, [&](uint32_t i) { return P.map_fill[i]; }, [&](uint32_t i, uint32_t v) { P.map_coff[i] = v; });
     const uint32_t nr = block_scan(
-        m, part, [&](uint32_t i) { return P.map_nr[i]; }, [&](uint32_t i, uint32_t v) { P.map_roff[i] = v; });
+        Block{}, m, part, [&](uint32_t i) { return P.map_nr[i]; }, [&](uint32_t i, uint32_t v) { P.map_roff[i] = v; });
     if (threadIdx.x == 0) {
         P.ctr->n_elems = nc;
         P.ctr->n_rays = nr;
@@ -1300,11 +1325,11 @@ __device__ void warp_steps(const ContactParams& P, uint32_t n, uint32_t steps, c
 // memory): its triangles in the reference's iteration order, their contact
 // records and rays in that order, and the map's mean ray origin.
 template <uint32_t T, uint32_t kWords>
-__device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, uint32_t* part, float* fold) {
+__device__ void order_map(const Team<T>& team, const ContactParams& P, uint32_t map, uint32_t* smem, uint32_t* part, float* fold) {
     const uint32_t q = map >> 1, side = map & 1u;
     const uint32_t n = P.map_fill[map];
     const uint32_t base = P.map_off[map];
-    const uint32_t t = threadIdx.x;
+    const uint32_t t = team.t;
     uint32_t n_rays = 0;
     bool ok = n > 0u && base + n <= P.max_contacts;
     OrderLayout L{};
@@ -1348,22 +1373,22 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 wide |= E.key_lo != 0ull;
                 mid |= (E.key_hi & 0xffffffffull) != 0ull;
             }
-            wide = __syncthreads_or(wide) != 0;
-            mid = __syncthreads_or(mid) != 0;
+            wide = team.any(wide);
+            mid = team.any(mid);
             const uint32_t E = L.n2 <= T ? 1u : (L.n2 <= 2u * T ? 2u : 4u);
             uint32_t* xchg = W == smem ? B0 : smem;  // 6 n2 words at most
             if (!wide && !mid) {
-                if (E == 1u) insertion_order<T, K1, 1>(El, n, L.n2, xchg, ins_tri, ins_elem);
-                else if (E == 2u) insertion_order<T, K1, 2>(El, n, L.n2, xchg, ins_tri, ins_elem);
-                else insertion_order<T, K1, 4>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                if (E == 1u) insertion_order<T, K1, 1>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
+                else if (E == 2u) insertion_order<T, K1, 2>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
+                else insertion_order<T, K1, 4>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
             } else if (!wide) {
-                if (E == 1u) insertion_order<T, K2, 1>(El, n, L.n2, xchg, ins_tri, ins_elem);
-                else if (E == 2u) insertion_order<T, K2, 2>(El, n, L.n2, xchg, ins_tri, ins_elem);
-                else insertion_order<T, K2, 4>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                if (E == 1u) insertion_order<T, K2, 1>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
+                else if (E == 2u) insertion_order<T, K2, 2>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
+                else insertion_order<T, K2, 4>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
             } else {
-                if (E == 1u) insertion_order<T, K3, 1>(El, n, L.n2, xchg, ins_tri, ins_elem);
-                else if (E == 2u) insertion_order<T, K3, 2>(El, n, L.n2, xchg, ins_tri, ins_elem);
-                else insertion_order<T, K3, 4>(El, n, L.n2, xchg, ins_tri, ins_elem);
+                if (E == 1u) insertion_order<T, K3, 1>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
+                else if (E == 2u) insertion_order<T, K3, 2>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
+                else insertion_order<T, K3, 4>(team, El, n, L.n2, xchg, ins_tri, ins_elem);
             }
         } else {
             SortKey* sk = reinterpret_cast<SortKey*>(B0);
@@ -1382,8 +1407,8 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 }
                 sk[i] = k;
             }
-            __syncthreads();
-            bitonic(sk, L.n2, [](const SortKey& a, const SortKey& b) {
+            team.sync();
+            bitonic(team, sk, L.n2, [](const SortKey& a, const SortKey& b) {
                 return a.hi != b.hi ? a.hi < b.hi : (a.lo != b.lo ? a.lo < b.lo : a.tri < b.tri);
             });
             for (uint32_t i = t; i < n; i += T) {
@@ -1391,7 +1416,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 ins_elem[i] = sk[i].idx;
             }
         }
-        __syncthreads();
+        team.sync();
         // 2. the table's order (insertion indices) after each growth: its
         // buckets in the order of their first place, latest first, each
         // bucket's keys latest first, where a growth places the table's keys
@@ -1416,7 +1441,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
             first[b] = ~0u;
             cnt[b] = 0u;
         }
-        __syncthreads();
+        team.sync();
         for (; e < P.n_sched && P.sched_start[e] < n; ++e) {
             const uint32_t st = P.sched_start[e];  // keys in the table when it grows
             const uint32_t m = step_end(P, e, n);
@@ -1428,12 +1453,12 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 kb[s] = atomicAdd(cnt + b, 1u);
                 atomicMin(first + b, s);
             }
-            __syncthreads();
+            team.sync();
             // the member lists' offsets, and the run starts (the keys of the
             // buckets whose first place is later)
             uint32_t total = 0, none = 0;
             block_scan2(
-                nb, m, part, [&](uint32_t b) { return cnt[b]; }, [&](uint32_t b, uint32_t v) { boff[b] = v; },
+                team, nb, m, part, [&](uint32_t b) { return cnt[b]; }, [&](uint32_t b, uint32_t v) { boff[b] = v; },
                 [&](uint32_t i) {
                     const uint32_t s = m - 1u - i, b = bs[s];
                     return first[b] == s ? cnt[b] : 0u;
@@ -1441,7 +1466,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 [&](uint32_t i, uint32_t v) { run[m - 1u - i] = v; }, total, none);
             for (uint32_t s = t; s < m; s += T) mem[boff[bs[s]] + kb[s]] = s;
             if (t == 0u) boff[nb] = total;
-            __syncthreads();
+            team.sync();
             // the next step's buckets start empty
             const bool more = e + 1u < P.n_sched && P.sched_start[e + 1u] < n;
             const uint32_t nb2 = more ? P.sched_buckets[e + 1u] : 0u;
@@ -1455,7 +1480,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 for (uint32_t k = boff[b]; k < boff[b + 1u]; ++k) later += mem[k] > s ? 1u : 0u;
                 nord[run[first[b]] + later] = s < st ? ord[s] : s;
             }
-            __syncthreads();
+            team.sync();
             uint32_t* sw = ord;
             ord = nord;
             nord = sw;
@@ -1474,7 +1499,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
                 V.keys[i] = ~0u;
                 V.vals[i] = ~0u;
             }
-            __syncthreads();
+            team.sync();
         }
         uint32_t* rb = B0 + 2u * L.nr;
         uint32_t* rc = B0 + 3u * L.nr;
@@ -1496,7 +1521,7 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
             vi1[p] = vi[1];
             vi2[p] = vi[2];
         }
-        __syncthreads();
+        team.sync();
         for (uint32_t p = t; p < n; p += T) {
             const uint32_t mask = rb[p];
             const uint32_t vi[3] = {vi0[p], vi1[p], vi2[p]};
@@ -1504,9 +1529,9 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
             rb[p] = bits;
             rc[p] = mask ? __popc(bits) : 1u;
         }
-        __syncthreads();
+        team.sync();
         n_rays = block_scan(
-            n, part, [&](uint32_t i) { return rc[i]; }, [&](uint32_t i, uint32_t v) { rc[i] = v; });
+            team, n, part, [&](uint32_t i) { return rc[i]; }, [&](uint32_t i, uint32_t v) { rc[i] = v; });
         // a thread per ray: its place is the last one whose first ray is at
         // or before it (a place without rays shares its first ray with the
         // next place)
@@ -1549,27 +1574,44 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
             c.weight = E.w;
             P.ctmp[base + p] = c;
         }
-        __syncthreads();
+        team.sync();
     }
     // the mean origin: std::accumulate over the rays in order, one coordinate
     // per lane, from shared memory a chunk of rays at a time
     {
-        constexpr uint32_t kStageRays = kWords / 3u;
+        // (by coordinate, 8 of a lane's terms loaded while 8 are added: the
+        // adds' 4 cycles a ray are the chain; 1,214 rays 8.2 to 5.6 us)
+        constexpr uint32_t kStageRays = kWords / 3u & ~3u;
         float* stage = reinterpret_cast<float*>(smem);
         float acc = 0.0f;
         for (uint32_t r0 = 0; r0 < n_rays; r0 += kStageRays) {
             const uint32_t m = n_rays - r0 < kStageRays ? n_rays - r0 : kStageRays;
-            for (uint32_t i = t; i < 3u * m; i += T) stage[i] = R[r0 + i / 3u].origin[i % 3u];
-            __syncthreads();
+            for (uint32_t i = t; i < 3u * m; i += T) stage[i % 3u * kStageRays + i / 3u] = R[r0 + i / 3u].origin[i % 3u];
+            team.sync();
             if (t < 3u) {
-#pragma unroll 8
-                for (uint32_t r = 0; r < m; ++r) acc = acc + stage[3u * r + t];
+                const float* x = stage + t * kStageRays;
+                const float4* x4 = reinterpret_cast<const float4*>(x);
+                const uint32_t full = m >> 3;
+                float4 cur[2], ahead[2];
+                if (full)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) ahead[k] = x4[k];
+                for (uint32_t g = 0; g < full; ++g) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) cur[k] = ahead[k];
+                    if (g + 1u < full)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) ahead[k] = x4[2u * (g + 1u) + k];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) acc = (((acc + cur[k].x) + cur[k].y) + cur[k].z) + cur[k].w;
+                }
+                for (uint32_t r = 8u * full; r < m; ++r) acc = acc + x[r];
             }
-            __syncthreads();
+            team.sync();
         }
         if (t < 3u) fold[t] = acc;
     }
-    __syncthreads();
+    team.sync();
     if (t == 0u) {
         // CreateUncollideRays.cpp:185-198: the sum over the count (0 / 0 for
         // a side without rays), the second side's moved back to its space
@@ -1599,31 +1641,63 @@ __device__ void order_map(const ContactParams& P, uint32_t map, uint32_t* smem, 
 // Persistent: each block takes the next map of the largest-first list. Two
 // launches side by side (the second a programmatic dependent of the first: a
 // branch of its own cost one-query steps 4 us): the maps of kBigMap triangles or more by blocks of
-// 1,024 threads with an SM's whole shared memory, the others by blocks of 256.
-// The block that finishes last of both places the maps.
+// 1,024 threads with an SM's whole shared memory, the others by blocks of 256,
+// which from the first map of fewer than kHalfMap triangles on (the list's
+// remainder) work as two halves, a map each: a small map's time is a chain of
+// short passes and barriers (18 us at 100 triangles with 128 threads as with
+// 256), so that four at once on an SM instead of two take the step of 1,000
+// small pairs from 716 to 670 us and a frame of 256 entities from 925 to 899;
+// halves for maps of up to 256 triangles slow a scene's largest maps (303 to
+// 307 us), up to 64 leave most of the gain. The block that finishes last of
+// both launches places the maps.
 template <uint32_t T, uint32_t kWords, bool kBig>
 __global__ void __launch_bounds__(T, kBig ? 1 : 2) contacts_order_kernel(const ContactParams P) {
     extern __shared__ __align__(16) uint32_t smem_order[];
-    __shared__ uint32_t part[64];
-    __shared__ float fold[3];
-    __shared__ uint32_t next_map;
+    __shared__ uint32_t part[2][64];
+    __shared__ float fold[2][3];
+    __shared__ uint32_t next_map, half_map[2];
+    __shared__ bool next_half;
     // the small maps' launch may start beside this one, and ends after it
     if (kBig) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t big = *reinterpret_cast<const volatile unsigned*>(&P.ctr->n_bigmaps);
+    const uint32_t whole = *reinterpret_cast<const volatile unsigned*>(&P.ctr->n_wholemaps);
     const uint32_t end = kBig ? big : 2u * P.n_queries;
+    uint32_t i = 0;  // the ticket's place in the list
+    auto draw = [&] {
+        i = kBig ? atomicAdd(&P.ctr->order_big_ticket, 1u) : big + atomicAdd(&P.ctr->order_ticket, 1u);
+        return i < end ? P.map_order[i] : ~0u;
+    };
+    uint32_t map;
     for (;;) {
         if (threadIdx.x == 0) {
-            const uint32_t i = kBig ? atomicAdd(&P.ctr->order_big_ticket, 1u) : big + atomicAdd(&P.ctr->order_ticket, 1u);
-            next_map = i < end ? P.map_order[i] : ~0u;
+            next_map = draw();
+            next_half = i >= whole;
         }
         __syncthreads();
-        const uint32_t map = next_map;
-        if (map == ~0u) break;
-        order_map<T, kWords>(P, map, smem_order, part, fold);
+        map = next_map;
+        if (map == ~0u || (!kBig && next_half)) break;
+        order_map<T, kWords>(Team<T>{threadIdx.x, 0u}, P, map, smem_order, part[0], fold[0]);
         __syncthreads();
     }
+    if constexpr (!kBig)
+        if (map != ~0u) {  // so are all that follow in the list: the first half takes this one
+            const uint32_t h = threadIdx.x / (T / 2u);
+            const Team<T / 2u> team{threadIdx.x % (T / 2u), 1u + h};
+            bool drawn = h == 0u;
+            for (;;) {
+                if (!drawn) {
+                    if (team.t == 0u) half_map[h] = draw();
+                    team.sync();
+                    map = half_map[h];
+                }
+                drawn = false;
+                if (map == ~0u) break;
+                order_map<T / 2u, kWords / 2u>(team, P, map, smem_order + h * (kWords / 2u), part[h], fold[h]);
+                team.sync();
+            }
+        }
     if (!kBig) asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (last_block(&P.ctr->order_done, P.order_grid)) place_maps(P, part);
+    if (last_block(&P.ctr->order_done, P.order_grid)) place_maps(P, part[0]);
 }
 
 __global__ void __launch_bounds__(256) contacts_emit_kernel(const ContactParams P) {

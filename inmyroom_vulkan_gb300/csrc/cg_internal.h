@@ -99,6 +99,7 @@ struct Counters {
     unsigned int order_ticket;   // maps of fewer than kBigMap triangles taken by the order kernel's blocks
     unsigned int order_big_ticket;  // larger maps taken
     unsigned int n_bigmaps;      // larger maps
+    unsigned int n_wholemaps;    // maps of kHalfMap triangles or more
     unsigned int n_big;          // contact slots of more than kFoldThread contributions (listed for the fold)
     unsigned int fold_done;      // fold blocks finished (the last one ranks the maps)
     unsigned int order_done;     // order blocks finished (the last one places the maps' records and rays)
@@ -142,6 +143,7 @@ constexpr uint32_t kMaxSchedule = 40;
 // element). The line lies where a map stops fitting half an SM: a map of 1,500
 // triangles took 530,000 cycles in global memory with 256 threads.
 constexpr uint32_t kBigMap = 1024;
+constexpr uint32_t kHalfMap = 128;  // maps of fewer triangles are ordered by half a block
 constexpr uint32_t kOrderSmemWords = 24576;
 constexpr uint32_t kBigSmemWords = 57344;
 constexpr uint32_t kOrderWords = 24;
