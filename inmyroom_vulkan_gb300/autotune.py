@@ -4,12 +4,13 @@ Picks, for one batch of queries on one context, the launch settings of the
 persistent traversal and the narrow phase that give the shortest device time:
 
   queue depth      queue_capacity (node pairs the global work queue holds)
-                   and donate_min (the stack depth above which a warp hands
-                   node pairs to idle warps)
+                   and donate_min (the stack depth per warp above which a
+                   worker block hands node pairs to idle ones)
   warps            warps_per_block and blocks_per_sm of the persistent
-                   traversal (lanes per node pair are picked per step by the
-                   kernel itself from the width of its work: 8, 16 or 32)
-  stack / tile     stack_entries (per-warp shared-memory node-pair stack) and
+                   traversal (which forms worker blocks of two or four of
+                   these warps and picks the lanes per node pair in each step
+                   from the width of its work)
+  stack / tile     stack_entries (node-pair stack of a pair of warps) and
                    leaf_flush (candidate leaf pairs a warp gathers before it
                    appends them to the narrow phase's list)
 

@@ -16,9 +16,9 @@
 //                 written out. As many launches as the largest possible list
 //                 needs (a list that needs fewer ends them at once)
 //
-// All of it is memory latency: 155,000 leaf pairs of 250 queries take about
-// 40 us where reading paths and pairs back and sorting them on the host took
-// 3.6 ms.
+// All of it is memory latency: 155,000 leaf pairs of 250 queries take 67 us
+// (tiles 32, merges 26) where reading paths and pairs back and sorting them on
+// the host took 3.6 ms.
 #include <cuda_runtime.h>
 
 #include "cg_internal.h"
