@@ -804,6 +804,7 @@ int cg_destroy(cg_ctx* c) {
     cudaFree(c->energy_table.dev);
     cudaFree(c->pose_scratch);
     cudaFree(c->vgrad);
+    cudaFree(c->skin);
     cudaFree(c->shoot);
     cudaFree(c->broad);
     cudaFree(c->frame);
@@ -1421,7 +1422,7 @@ int cg_energy_backward(cg_ctx* c, const double* d_grad_energy, const cg_energy_s
     const uint32_t n = c->last_n;
     std::vector<EnergySide> sides(2ull * n);
     std::vector<uint32_t> deforming;
-    uint64_t total = 0;
+    uint64_t total = 0, joints = 0;
     uint32_t max_vertices = 0, max_joints = 0, max_targets = 0;
     const cg_energy_side* both[2] = {side_a, side_b};
     for (uint32_t k = 0; k < 2; ++k) {
@@ -1448,6 +1449,8 @@ int cg_energy_backward(cg_ctx* c, const double* d_grad_energy, const cg_energy_s
             deforming.push_back(k * n + q);
             max_vertices = std::max(max_vertices, e.d.n_vertices);
             max_joints = std::max(max_joints, e.d.n_joints);
+            e.skin_base = uint32_t(joints);
+            joints += e.d.n_groups ? e.d.n_joints : 0u;
             max_targets = std::max(max_targets, e.d.n_targets);
         }
     }
@@ -1473,6 +1476,17 @@ int cg_energy_backward(cg_ctx* c, const double* d_grad_energy, const cg_energy_s
         CG_CUDA(cudaMemset(c->vgrad, 0, sizeof(float) * 3u * total), "zero vertex gradients");
         c->vgrad_cap = 3u * total;
     }
+    if (joints > c->skin_cap) {
+        CG_CUDA(cudaStreamSynchronize(s), "skin matrix buffer");
+        cudaFree(c->skin);
+        c->skin = nullptr;
+        c->skin_cap = 0;
+        // without room the kernels form the matrices on the spot
+        if (cudaMalloc(&c->skin, sizeof(float) * 16u * joints) == cudaSuccess)
+            c->skin_cap = joints;
+        else
+            cudaGetLastError();
+    }
     std::vector<char> blob(sizeof(EnergySide) * sides.size() + sizeof(uint32_t) * deforming.size());
     std::memcpy(blob.data(), sides.data(), sizeof(EnergySide) * sides.size());
     std::memcpy(blob.data() + sizeof(EnergySide) * sides.size(), deforming.data(), sizeof(uint32_t) * deforming.size());
@@ -1485,6 +1499,7 @@ int cg_energy_backward(cg_ctx* c, const double* d_grad_energy, const cg_energy_s
     p.deforming = reinterpret_cast<const uint32_t*>(static_cast<const char*>(d_blob) + sizeof(EnergySide) * sides.size());
     p.n_deforming = uint32_t(deforming.size());
     p.vgrad = c->vgrad;
+    p.skin = joints && joints <= c->skin_cap && joints <= 0xffffffffull ? c->skin : nullptr;
     p.max_joints = max_joints;
     p.max_targets = max_targets;
     CG_CUDA(launch_energy_backward(p, c->energy_blocks, max_vertices, s), "energy adjoint kernels");

@@ -234,6 +234,8 @@ struct cg_ctx {
     uint64_t pose_scratch_cap = 0;
     float* vgrad = nullptr;                 // energy adjoint: per-vertex gradient, zero between calls
     uint64_t vgrad_cap = 0;
+    float* skin = nullptr;                  // energy adjoint: the deforming sides' skin matrices
+    uint64_t skin_cap = 0;                  // joints
     void* shoot = nullptr;                  // cg_shoot_rays: queries, rays, tags, per-ray results, deltas, flag
     size_t shoot_cap = 0;
     void* broad = nullptr;                  // cg_broad_phase: ids, globals, callbacks, projections, pairs, count

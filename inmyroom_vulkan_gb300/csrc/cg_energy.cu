@@ -380,14 +380,42 @@ __global__ void __launch_bounds__(256) energy_kernel(const EnergyParams P) {
     if (threadIdx.x == 0 && s != 0.0) atomicAdd(P.energy, s);
 }
 
+// The deforming sides' skin matrices (joint_matrix * inverse_bind), a thread
+// per entry, for the two kernels below. Formed on the spot (450 instructions
+// and 32 loads a vertex) they made vertex_grad take 56 us for 64 tubes in
+// contact; with the table it takes 40, and the table 4.
+__global__ void __launch_bounds__(256) skin_matrices_kernel(const EnergyParams P) {
+    const EnergySide& S = P.sides[P.deforming[blockIdx.y]];
+    const uint32_t e = blockIdx.x * 256u + threadIdx.x, j = e >> 4;
+    if (!S.d.n_groups || j >= S.d.n_joints) return;
+    P.skin[16ull * S.skin_base + e] = skin_entry(S.d.joint_matrices + 16ull * j, S.d.inverse_bind + 16ull * j, e & 15u);
+}
+
+__device__ __forceinline__ void skin_matrix(const EnergyParams& P, const EnergySide& S, uint32_t j, float* m) {
+    if (P.skin) {
+        const float4* M = reinterpret_cast<const float4*>(P.skin) + 4ull * (uint64_t(S.skin_base) + j);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float4 c = __ldg(M + k);
+            m[4 * k] = c.x, m[4 * k + 1] = c.y, m[4 * k + 2] = c.z, m[4 * k + 3] = c.w;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 16; ++i)
+            m[i] = skin_entry(S.d.joint_matrices + 16ull * j, S.d.inverse_bind + 16ull * j, i);
+    }
+}
+
 // The side's three vertices: recomputed from its view when it deforms, else
 // the stored triangle. False when a vertex index is outside the view.
-__device__ __forceinline__ bool side_vertices(const EnergySide& S, const uint32_t vi[3], float3 p[3]) {
+__device__ __forceinline__ bool side_vertices(const EnergyParams& P, const EnergySide& S, const uint32_t vi[3],
+                                              float3 p[3]) {
     if (S.d.n_vertices == 0) return true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         if (vi[k] >= S.d.n_vertices) return false;
-        const float4 v = deform_vertex(S.d, vi[k]);
+        const float4 v = skin_vertex(S.d, vi[k], morph_vertex(S.d, vi[k]),
+                                     [&](uint32_t j, float* m) { skin_matrix(P, S, j, m); });
         p[k] = make_float3(v.x, v.y, v.z);
     }
     return true;
@@ -400,7 +428,7 @@ __device__ __forceinline__ void add_vgrad(float* vgrad, uint32_t base, uint32_t 
     atomicAdd(p + 2, g.z);
 }
 
-__global__ void __launch_bounds__(256) vertex_grad_kernel(const EnergyParams P) {
+__global__ void __launch_bounds__(256, 3) vertex_grad_kernel(const EnergyParams P) {
     const unsigned long long n = stored_pairs(P);
     const float g = float(*P.grad_energy);
     for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) {
@@ -414,7 +442,7 @@ __global__ void __launch_bounds__(256) vertex_grad_kernel(const EnergyParams P) 
         uint32_t va[3], vb[3];
         load_tri(P.tris, __ldg(&Q.tri_base_a) + pr.tri_a, pa, va);
         load_tri(P.tris, __ldg(&Q.tri_base_b) + pr.tri_b, pb, vb);
-        if (!side_vertices(SA, va, pa) || !side_vertices(SB, vb, pb)) continue;
+        if (!side_vertices(P, SA, va, pa) || !side_vertices(P, SB, vb, pb)) continue;
         const Mat4 M = pair_matrix(Q);
 #pragma unroll
         for (int k = 0; k < 3; ++k) pb[k] = xform(M, pb[k], 1.0f);
@@ -530,9 +558,7 @@ __global__ void __launch_bounds__(256) skin_adjoint_kernel(const EnergyParams P)
 #pragma unroll
                         for (int i = 0; i < 16; ++i) m[i] = Ms[16u * j + i];
                     } else {
-#pragma unroll
-                        for (uint32_t i = 0; i < 16; ++i)
-                            m[i] = skin_entry(D.joint_matrices + 16ull * j, D.inverse_bind + 16ull * j, i);
+                        skin_matrix(P, ES, j, m);
                     }
 #pragma unroll
                     for (int cc = 0; cc < 4; ++cc)  // S_j^T (w g)
@@ -632,12 +658,15 @@ cudaError_t launch_energy(const EnergyParams& p, uint32_t blocks, cudaStream_t s
 }
 
 cudaError_t launch_energy_backward(const EnergyParams& p, uint32_t blocks, uint32_t max_vertices, cudaStream_t s) {
+    if (p.skin && p.n_deforming)
+        skin_matrices_kernel<<<dim3((p.max_joints + 15u) / 16u, p.n_deforming), 256, 0, s>>>(p);
     vertex_grad_kernel<<<blocks, 256, 0, s>>>(p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || p.n_deforming == 0 || max_vertices == 0) return e;
     EnergyParams q = p;
-    // skin matrices staged in shared memory up to kSkinStagedJoints joints
-    q.skin_in_smem = p.max_joints <= kSkinStagedJoints ? 1u : 0u;
+    // skin matrices without a table staged in shared memory up to
+    // kSkinStagedJoints joints
+    q.skin_in_smem = !p.skin && p.max_joints <= kSkinStagedJoints ? 1u : 0u;
     const size_t smem = sizeof(float) * ((q.skin_in_smem ? 28u : 12u) * p.max_joints + p.max_targets);
     skin_adjoint_kernel<<<dim3((max_vertices + 255u) / 256u, p.n_deforming), 256, smem, s>>>(q);
     return cudaGetLastError();

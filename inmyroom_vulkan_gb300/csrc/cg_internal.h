@@ -409,7 +409,7 @@ cudaError_t launch_pose_backward(const PoseParams& p, cudaStream_t s);
 struct EnergySide {
     DeformParams d;      // d.n_vertices == 0: the side is static
     uint32_t grad_base;  // first vertex of this side in the vertex-gradient buffer
-    uint32_t pad;
+    uint32_t skin_base;  // first joint of this side in EnergyParams::skin
     float* grad_joint;   // [joint_stride][16], rows 0-2 written
     float* grad_morph;   // [n_targets]
 };
@@ -426,6 +426,7 @@ struct EnergyParams {
     const EnergySide* sides;      // [2 * n_queries]: side A of every query, then side B
     const uint32_t* deforming;    // indices into sides of the deforming ones
     float* vgrad;                 // [sum of deforming sides' n_vertices][3], zero between calls
+    float* skin;                  // [sum of deforming sides' joints][16]: their skin matrices; null: formed on the spot
     uint32_t max_joints, max_targets;
     uint32_t skin_in_smem;        // set by the launcher
 };
