@@ -112,7 +112,7 @@ __device__ __forceinline__ void warp_extreme(Ext& e, bool lo) {
 }
 
 // A level's kernels are launched as programmatic dependents, each on the one
-// before it in the stream (next, below). after_all waits until that one has
+// before it in the stream (launch_next). after_all waits until that one has
 // finished; with B.early the blocks of the next one may start as soon as this
 // one's all have, so that its launch runs beside this kernel. That is for next
 // kernels of a block an SM at most, or of a block per node: a larger grid's
@@ -1463,25 +1463,6 @@ cudaError_t build_smem_limit() {
                                 int(sizeof(ReplayBig)));
 }
 
-namespace {
-// A launch as a programmatic dependent of the one before it in the stream.
-template <class... P, class... A>
-cudaError_t next(void (*kernel)(P...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t s, const A&... a) {
-    cudaLaunchAttribute early{};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(a)...), last = cudaGetLastError();
-    return e != cudaSuccess ? e : last;
-}
-}  // namespace
-
 cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStream_t s) {
     if (p.hi <= p.lo) return cudaSuccess;
     const uint32_t width = p.hi - p.lo;
@@ -1498,7 +1479,7 @@ cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStre
     // after a kernel whose next has `then` blocks (1: a block per node)
     auto run = [&](void (*kernel)(const BuildParams), uint32_t n, uint32_t threads, size_t smem, uint32_t then) {
         q.early = then <= sm_count;
-        if (e == cudaSuccess) e = next(kernel, n, threads, smem, s, q);
+        if (e == cudaSuccess) e = launch_next(kernel, n, threads, smem, s, q);
     };
     // of a stage the smallest nodes' kernel first: it is the one that waits
     run(build_sums_kernel, g_sum, 128, 0, p.n_big ? 1u : g_tri);
@@ -1522,7 +1503,7 @@ cudaError_t launch_build_level(const BuildParams& p, uint32_t sm_count, cudaStre
     }
     if (lanes) {
         q.early = g_tri <= sm_count;
-        if (e == cudaSuccess) e = next(build_eig_group_kernel, g_eig, 128, 0, s, q, lanes);
+        if (e == cudaSuccess) e = launch_next(build_eig_group_kernel, g_eig, 128, 0, s, q, lanes);
     } else {
         run(build_eig_kernel, g_node, 128, 0, g_tri);
     }
@@ -1568,7 +1549,7 @@ cudaError_t launch_build_inner(const BuildParams& p, BuildFlat* flat, uint32_t s
     BuildParams q = p;
     const uint32_t blocks = grid_of(p.hi - p.lo, sm_count);
     q.early = blocks <= sm_count;
-    return next(build_inner_kernel, blocks, 128, 0, s, q, flat);
+    return launch_next(build_inner_kernel, blocks, 128, 0, s, q, flat);
 }
 
 cudaError_t launch_build_order(const BuildParams& p, BuildFlat* flat, uint32_t n_roots, uint32_t sm_count,
@@ -1577,7 +1558,7 @@ cudaError_t launch_build_order(const BuildParams& p, BuildFlat* flat, uint32_t n
     BuildParams q = p;
     const uint32_t blocks = grid_of(p.hi - p.lo, sm_count);
     q.early = blocks <= sm_count;
-    return next(build_order_kernel, blocks, 128, 0, s, q, flat, n_roots);
+    return launch_next(build_order_kernel, blocks, 128, 0, s, q, flat, n_roots);
 }
 
 cudaError_t launch_build_emit(const BuildParams& p, const BuildInput& in, const BuildFlat* flat,

@@ -1902,17 +1902,7 @@ cudaError_t launch_contacts(const ContactParams& p_in, uint32_t grid, uint32_t f
     const uint32_t small = maps < order_grid ? maps : order_grid, big = maps < big_grid ? maps : big_grid;
     p.order_grid = small + big;
     order_big<<<big, 1024, kBigSmemWords * sizeof(uint32_t), s>>>(p);
-    cudaLaunchAttribute beside{};
-    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    beside.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(small);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = kOrderSmemWords * sizeof(uint32_t);
-    cfg.stream = s;
-    cfg.attrs = &beside;
-    cfg.numAttrs = 1;
-    if ((e = cudaLaunchKernelEx(&cfg, order_small, p)) != cudaSuccess) return e;
+    if ((e = launch_next(order_small, small, 256, kOrderSmemWords * sizeof(uint32_t), s, p)) != cudaSuccess) return e;
     contacts_emit_kernel<<<maps < grid ? maps : grid, 256, 0, s>>>(p);
     return cudaGetLastError();
 }

@@ -205,6 +205,27 @@ struct ContactParams {
 
 cudaError_t launch_contacts(const ContactParams& p, uint32_t grid, uint32_t fold_grid, uint32_t order_grid,
                             uint32_t big_grid, cudaStream_t s, cudaStream_t branch, cudaEvent_t ev_fork, cudaEvent_t ev_join);
+// A launch as a programmatic dependent of the one before it in the stream: its
+// blocks may start when that one's have ended or said so
+// (griddepcontrol.launch_dependents), and wait (griddepcontrol.wait) for its
+// results.
+template <class... P, class... A>
+cudaError_t launch_next(void (*kernel)(P...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t s,
+                        const A&... a) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(a)...), last = cudaGetLastError();
+    return e != cudaSuccess ? e : last;
+}
+
 cudaError_t contacts_order_occupancy(int* blocks_per_sm);
 cudaError_t contacts_fold_occupancy(int* blocks_per_sm);
 
@@ -595,7 +616,7 @@ cudaError_t launch_frame_split(const FrameParams& p, cudaStream_t s);
 
 // Kernel launchers (cg_kernels.cu).
 cudaError_t launch_pack(const cg_query* in, uint32_t n, const DevTree* trees, uint32_t n_trees, const float4* recs,
-                        PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap, cudaStream_t s);
+                        PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap, bool early, cudaStream_t s);
 cudaError_t launch_init(Counters* ctr, unsigned int* ready, uint32_t slot_alloc, uint32_t n_queries,
                         unsigned int* trace, cudaStream_t s);
 cudaError_t launch_traverse(const TraverseParams& p, uint32_t blocks, uint32_t warps_per_block, cudaStream_t s);
