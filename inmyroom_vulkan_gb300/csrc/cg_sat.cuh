@@ -27,8 +27,11 @@
 // The filter's own margin, three chained roundings per triple product, a
 // rounded d and four sums, is within 9u W |x||y| of it. kSatK = 32u covers the
 // two together with room for the bound's own rounding; the added constant
-// covers products that underflow. A NaN or an overflow makes every comparison
-// with the bound false: the axis stays open.
+// covers products that underflow. A NaN makes every comparison with the bound
+// false: the axis stays open. An infinity does not (the bound is a 2^-19th of
+// products that the margin is a sum of, and may be finite beside it), so from
+// W = 1e12 on, NaN included, all axes stay open: below it no product, sum or
+// interval end of either side exceeds 8 W^3 = 8e36.
 #pragma once
 
 #include <cstdint>
@@ -58,6 +61,7 @@ __device__ __forceinline__ bool sat_axis(const Box& a, const Box& b, uint32_t k)
 
 constexpr float kSatK = 32.0f * 0x1p-24f;
 constexpr float kSatTiny = 0x1p-120f;
+constexpr float kSatMax = 1e12f;
 
 __device__ __forceinline__ float norm1_3(float3 p) { return (fabsf(p.x) + fabsf(p.y)) + fabsf(p.z); }
 __device__ __forceinline__ float fdot(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
@@ -152,8 +156,9 @@ __device__ __forceinline__ bool sat_filter(const SatBox& x, const SatBox& y, uns
             axis(6 + 3 * i + j, (g[i1][j] + g[i2][j]) + (h[i][j1] + h[i][j2]), fdot(ye[j], e), fmaf(ki, yl[j], T));
         }
     }
-    open = m;
-    return sep;
+    const bool sane = W < kSatMax;
+    open = sane ? m : 0x7fffu;
+    return sane && sep;
 }
 
 }  // namespace cg
