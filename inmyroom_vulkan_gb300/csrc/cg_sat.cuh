@@ -62,6 +62,7 @@ __device__ __forceinline__ bool sat_axis(const Box& a, const Box& b, uint32_t k)
 constexpr float kSatK = 32.0f * 0x1p-24f;
 constexpr float kSatTiny = 0x1p-120f;
 constexpr float kSatMax = 1e12f;
+constexpr float kSurfaceTiny = 0x1p-70f, kSurfaceMax = 1e18f;
 
 __device__ __forceinline__ float norm1_3(float3 p) { return (fabsf(p.x) + fabsf(p.y)) + fabsf(p.z); }
 __device__ __forceinline__ float fdot(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
@@ -105,10 +106,15 @@ __device__ __forceinline__ SatBox sat_box(const Box& b) {
 // Paralgram::GetSurface of the box (cg::surface) from its normals, and how far
 // that can be from the reference's FP32 value: each normal's components are
 // within 2u, as the reference's are, of exact ones bounded by its edges'
-// 1-norms; the norms and their sum add at most 8u.
+// 1-norms; the norms and their sum add at most 8u. Squares that underflow put
+// a squared norm off by up to 2^-148 and its root by 2^-74: six roots, the
+// reference's among them, doubled, by less than kSurfaceTiny. Where squares
+// may overflow (the products of 1-norms bound the normals) the error has no
+// limit: one side's sum may be finite beside an infinite one.
 __device__ __forceinline__ float sat_surface(const SatBox& s, float& err) {
     const float q = norm_approx(s.nu) + norm_approx(s.nv) + norm_approx(s.nw);
-    err = fmaf(kSatK, fmaf(s.lu, s.lv, fmaf(s.lu, s.lw, s.lv * s.lw)), kSatTiny);
+    const float l = fmaf(s.lu, s.lv, fmaf(s.lu, s.lw, s.lv * s.lw));
+    err = l < kSurfaceMax ? fmaf(kSatK, l, kSurfaceTiny) : HUGE_VALF;
     return 2.0f * q;
 }
 
