@@ -1692,8 +1692,14 @@ __global__ void __launch_bounds__(T, kBig ? 1 : 2) contacts_order_kernel(const C
     __shared__ float fold[2][3];
     __shared__ uint32_t next_map, half_map[2];
     __shared__ bool next_half;
-    // the small maps' launch may start beside this one, and ends after it
-    if (kBig) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // The small maps' launch may start beside this one, and ends after it. Its
+    // blocks start once all of this one's have, that is after all kernels
+    // before this one have finished; as it waits for nothing before it reads
+    // what those wrote, it reads that past L1's old lines.
+    if constexpr (kBig)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    else
+        __threadfence();
     const uint32_t big = *reinterpret_cast<const volatile unsigned*>(&P.ctr->n_bigmaps);
     const uint32_t whole = *reinterpret_cast<const volatile unsigned*>(&P.ctr->n_wholemaps);
     const uint32_t end = kBig ? big : 2u * P.n_queries;
