@@ -391,7 +391,7 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
     CG_CUDA(launch_init(c->d_ctr, c->d_ready, c->slot_alloc, n, trace, s), "init kernel");
     const uint32_t leaf_cap = uint32_t(std::min<uint64_t>(c->cfg.max_leaf_pairs, 0xffffffffull));
     CG_CUDA(launch_pack(d_queries, n, c->d_trees, uint32_t(c->trees.size()), c->recs.ptr, c->d_packed, c->d_ctr,
-                        c->d_leaf_list, leaf_cap, true, s),
+                        c->d_leaf_list, leaf_cap, s),
             "pack kernel");
     TraverseParams p{};
     p.q = c->d_packed;
@@ -1636,7 +1636,7 @@ extern "C" int cg_collide_static(cg_ctx* c, const cg_query* d_queries, uint32_t 
 
     CG_CUDA(launch_init(ctr, ready, kStaticSlots, n, nullptr, s), "init kernel");
     CG_CUDA(launch_pack(d_queries, n, c->d_trees, uint32_t(c->trees.size()), c->recs.ptr, packed, ctr, leaf_list,
-                        CG_STATIC_MAX_LEAF_PAIRS, false, s),
+                        CG_STATIC_MAX_LEAF_PAIRS, s),
             "pack kernel");
     TraverseParams p{};
     p.q = packed;

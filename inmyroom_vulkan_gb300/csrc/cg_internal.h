@@ -616,7 +616,7 @@ cudaError_t launch_frame_split(const FrameParams& p, cudaStream_t s);
 
 // Kernel launchers (cg_kernels.cu).
 cudaError_t launch_pack(const cg_query* in, uint32_t n, const DevTree* trees, uint32_t n_trees, const float4* recs,
-                        PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap, bool early, cudaStream_t s);
+                        PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap, cudaStream_t s);
 cudaError_t launch_init(Counters* ctr, unsigned int* ready, uint32_t slot_alloc, uint32_t n_queries,
                         unsigned int* trace, cudaStream_t s);
 cudaError_t launch_traverse(const TraverseParams& p, uint32_t blocks, uint32_t warps_per_block, cudaStream_t s);

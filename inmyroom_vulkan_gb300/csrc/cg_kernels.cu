@@ -769,11 +769,7 @@ __global__ void __launch_bounds__(256, 3) narrow_kernel(const NarrowParams P) {
 // One thread per query: packs the relative matrix and runs the root pair the
 // way the traversal runs every pair (SAT, then the descent rule), so that the
 // query enters the work queue as its first item; a leaf-leaf root goes
-// straight to the leaf-pair list. A chain of dependent loads and one box test;
-// launched as init's programmatic dependent it overlaps that kernel up to its
-// first write of the counters (a one-pair step 176.6 to 175.1 us, the scene 336
-// to 334; the same for the contact kernels' lists slowed the scene's branch by
-// 10 us).
+// straight to the leaf-pair list.
 __global__ void pack_kernel(const cg_query* in, uint32_t n, const DevTree* trees, uint32_t n_trees,
                             const float4* recs, PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -791,7 +787,6 @@ __global__ void pack_kernel(const cg_query* in, uint32_t n, const DevTree* trees
     p.tree_b = Q.tree_b;
     const bool ok = Q.tree_a < n_trees && Q.tree_b < n_trees && trees[Q.tree_a].live && trees[Q.tree_b].live;
     if (!ok) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
         atomicOr(&ctr->error, ERR_BAD_QUERY);
         out[i] = p;
         return;
@@ -804,14 +799,12 @@ __global__ void pack_kernel(const cg_query* in, uint32_t n, const DevTree* trees
     const Rec A = load_rec(recs, ra);
     const Rec B = load_rec(recs, rb);
     const Box bb = xform_box(M, B.box);
-    const bool hit = sat(A.box, bb);
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the counters are reset by now
     {
         // one atomic per group of converged lanes
         const unsigned m = __activemask();
         if ((threadIdx.x & 31u) == unsigned(__ffs(m) - 1)) atomicAdd(&ctr->node_pairs, (unsigned long long)__popc(m));
     }
-    if (hit) {
+    if (sat(A.box, bb)) {
         const bool la = (A.meta & kLeafFlag) != 0;
         const bool lb = (B.meta & kLeafFlag) != 0;
         if (la && lb) {
@@ -832,8 +825,6 @@ __global__ void pack_kernel(const cg_query* in, uint32_t n, const DevTree* trees
 // counters), and the trace when it is kept.
 __global__ void init_kernel(Counters* ctr, unsigned int* ready, uint32_t slot_alloc, uint32_t n_queries,
                             unsigned int* trace) {
-    // the pack kernel waits for this one only before it counts
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ uint32_t used;
     if (threadIdx.x == 0) used = min(ctr->tail, slot_alloc);
     __syncthreads();
@@ -865,11 +856,9 @@ __global__ void surfaces_kernel(float4* recs, uint32_t first, uint32_t n_recs) {
 }
 
 cudaError_t launch_pack(const cg_query* in, uint32_t n, const DevTree* trees, uint32_t n_trees, const float4* recs,
-                        PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap, bool early, cudaStream_t s) {
+                        PackedQuery* out, Counters* ctr, uint4* leaf_list, uint32_t leaf_cap, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    const uint32_t blocks = (n + 127) / 128;
-    if (early) return launch_next(pack_kernel, blocks, 128, 0, s, in, n, trees, n_trees, recs, out, ctr, leaf_list, leaf_cap);
-    pack_kernel<<<blocks, 128, 0, s>>>(in, n, trees, n_trees, recs, out, ctr, leaf_list, leaf_cap);
+    pack_kernel<<<(n + 127) / 128, 128, 0, s>>>(in, n, trees, n_trees, recs, out, ctr, leaf_list, leaf_cap);
     return cudaGetLastError();
 }
 
