@@ -57,7 +57,7 @@ typedef struct cg_config {
     uint32_t queue_capacity;   /* node pairs the global work queue can hold (in chunks of 32) */
     uint32_t warps_per_block;  /* persistent traversal kernel shape; 0 = tuned default */
     uint32_t blocks_per_sm;    /* 0 = as many as fit */
-    uint32_t stack_entries;    /* shared-memory node-pair stack of a pair of warps, power of two (256..4096) */
+    uint32_t stack_entries;    /* shared-memory node-pair stack per warp, power of two (256..4096) */
     uint32_t donate_min;       /* warps donate work to idle warps only above this stack size per warp */
     uint32_t leaf_flush;       /* leaf pairs buffered per traversal warp before they go to the list (1..33) */
     uint32_t wait_limit_ms;    /* limit of every device-side wait */

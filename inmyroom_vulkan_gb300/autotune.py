@@ -10,7 +10,7 @@ persistent traversal and the narrow phase that give the shortest device time:
                    traversal (which forms worker blocks of two or four of
                    these warps and picks the lanes per node pair in each step
                    from the width of its work)
-  stack / tile     stack_entries (node-pair stack of a pair of warps) and
+  stack / tile     stack_entries (per-warp shared-memory node-pair stack) and
                    leaf_flush (candidate leaf pairs a warp gathers before it
                    appends them to the narrow phase's list)
 

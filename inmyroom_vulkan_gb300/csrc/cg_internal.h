@@ -321,12 +321,12 @@ struct TraverseParams {
 };
 
 
-// Entries of the deque of a worker block of W (1, 2 or 4) warps. With
-// stack_cap >= 256 it is at least 64 W + 64, so that a step's pushes fit after
-// a forced donation.
-__host__ __device__ inline uint32_t deque_entries(uint32_t stack_cap, uint32_t W) {
-    return W >= 4u ? 2u * stack_cap : stack_cap;
-}
+// Entries of the deque of a worker block of W (1, 2 or 4) warps: stack_cap for
+// each warp (the setting is per warp, as donate_min is). With half of that for
+// a pair of warps, deques filled up earlier and forced donations used up the
+// queue's slots: 2,000 uneven queries needed a queue_capacity of 65,536 where
+// 2,048 holds them so.
+__host__ __device__ inline uint32_t deque_entries(uint32_t stack_cap, uint32_t W) { return stack_cap * W; }
 __host__ __device__ inline uint32_t traverse_smem_words(uint32_t stack_cap, uint32_t W) {
     return 3u * deque_entries(stack_cap, W) + 4u * kLeafCap * W;
 }

@@ -883,7 +883,14 @@ namespace {
 // 59, 51, 48, 47; 64 of these 85, 67, 58, 64; 150 queries of 2 x 20,000 213,
 // 180, 190, 202; the 256-entity scene 131, 103, 110, 119; 10,000 uneven
 // queries 1310, 1288, 1392, 1587.
-uint32_t worker_warps(uint32_t n_queries, uint32_t total_warps) {
+// With the smallest stacks (256 entries) a worker is one warp and takes one root
+// at a time: donations that a full stack forces are then the rule, and how many
+// of the queue's slots they take decides whether a launch fits its queue. Two
+// 32,768-triangle meshes fit 256 slots so and not 64; those of wider workers fit
+// 64, or, with half the entries per warp, need 512.
+constexpr uint32_t kPoolStack = 512;
+uint32_t worker_warps(uint32_t n_queries, uint32_t total_warps, uint32_t stack_cap) {
+    if (stack_cap < kPoolStack) return 1u;
     return uint64_t(n_queries) * 8u <= total_warps && total_warps >= 4u ? 4u : (total_warps >= 2u ? 2u : 1u);
 }
 constexpr uint32_t kStackMax = 4096;  // cg_config.stack_entries' limit
@@ -918,10 +925,13 @@ cudaError_t narrow_occupancy(uint32_t warps_per_block, int* blocks_per_sm) {
 
 cudaError_t launch_traverse(const TraverseParams& p_in, uint32_t blocks, uint32_t warps_per_block, cudaStream_t s) {
     TraverseParams p = p_in;
-    const uint32_t total = blocks * warps_per_block, W = worker_warps(p.n_queries, total), workers = total / W;
+    const uint32_t total = blocks * warps_per_block, W = worker_warps(p.n_queries, total, p.stack_cap),
+                   workers = total / W;
     p.donate_min *= W;
     // all roots start at once where they fit a step of the workers
-    p.root_batch = std::min(std::max((p.n_queries + workers - 1u) / workers, 1u), 32u * W);
+    p.root_batch = p.stack_cap < kPoolStack
+                       ? 1u
+                       : std::min(std::max((p.n_queries + workers - 1u) / workers, 1u), 32u * W);
     const size_t smem = size_t(traverse_smem_words(p.stack_cap, W)) * sizeof(uint32_t);
     traverse_kernel<<<workers, 32 * W, smem, s>>>(p);
     return cudaGetLastError();
