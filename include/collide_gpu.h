@@ -237,7 +237,8 @@ typedef struct cg_stats {
  * src/Geometry/OBBtree.cpp:414-476: the order of their paths from the root
  * pair, left before right), the exact vector ExecuteOBBtreesCollision
  * returns. Each leaf pair's path is found on the device; a path of 128 or
- * more splits makes the launch CG_ERR_OUTPUT_OVERFLOW. */
+ * more splits makes the launch CG_ERR_OUTPUT_OVERFLOW. The first such launch
+ * allocates 24 bytes of device memory per max_leaf_pairs. */
 #define CG_DFS_ORDER 128u
 
 /* Per-triangle contact record, the TriangleCandidateRays of

@@ -54,8 +54,7 @@ void free_buffers(cg_ctx* c) {
     cudaFree(c->d_ready);
     cudaFree(c->d_pairs);
     cudaFree(c->d_leafs);
-    for (void* p : {(void*)c->order.keys, (void*)c->order.key[0], (void*)c->order.key[1], (void*)c->order.place,
-                    (void*)c->order.index[0], (void*)c->order.index[1], (void*)c->order.queries})
+    for (void* p : {(void*)c->order.keys, (void*)c->order.place, (void*)c->order.index, (void*)c->order.queries})
         cudaFree(p);
     c->order = cg_ctx::LeafOrder{};
     cudaFree(c->d_trace);
@@ -456,8 +455,11 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
         op.place = kp.place;
         op.first = kp.count + c->cfg.max_queries;
         op.tile = op.first + c->cfg.max_queries;
-        for (int k = 0; k < 2; ++k) op.key[k] = c->order.key[k], op.index[k] = c->order.index[k];
         op.out = c->d_leafs;
+        op.key[0] = reinterpret_cast<ulonglong2*>(c->d_leafs);
+        op.key[1] = c->order.keys;
+        op.index[0] = c->order.index;
+        op.index[1] = c->order.place;
         CG_CUDA(launch_leaf_order(op, uint32_t(c->sm_count), s), "leaf-pair order kernels");
     }
     if (pairs_copy) {
@@ -609,10 +611,7 @@ int check_flags(cg_ctx* c, uint32_t flags) {
         if (!o.queries) {
             if (!o.keys) CG_CUDA(cudaMalloc(&o.keys, sizeof(ulonglong2) * m), "alloc leaf-pair keys");
             if (!o.place) CG_CUDA(cudaMalloc(&o.place, sizeof(uint32_t) * m), "alloc leaf-pair places");
-            for (int k = 0; k < 2; ++k) {
-                if (!o.key[k]) CG_CUDA(cudaMalloc(&o.key[k], sizeof(ulonglong2) * m), "alloc leaf-pair order");
-                if (!o.index[k]) CG_CUDA(cudaMalloc(&o.index[k], sizeof(uint32_t) * m), "alloc leaf-pair order");
-            }
+            if (!o.index) CG_CUDA(cudaMalloc(&o.index, sizeof(uint32_t) * m), "alloc leaf-pair order");
             CG_CUDA(cudaMalloc(&o.queries, sizeof(uint32_t) * (3ull * c->cfg.max_queries + 1u)), "alloc leaf-pair order");
         }
     }

@@ -140,10 +140,11 @@ struct cg_ctx {
     cg_tri_pair* d_pairs = nullptr;
     cg_leaf_pair* d_leafs = nullptr;
     // CG_DFS_ORDER, allocated on first use: each leaf pair's descent path and
-    // number within its query, the sort's two buffers, the queries' counts and places
+    // number within its query (the sort's second buffers, too), the sort's
+    // indexes, the queries' counts and places
     struct LeafOrder {
-        ulonglong2 *keys = nullptr, *key[2] = {nullptr, nullptr};
-        uint32_t *place = nullptr, *index[2] = {nullptr, nullptr}, *queries = nullptr;
+        ulonglong2* keys = nullptr;
+        uint32_t *place = nullptr, *index = nullptr, *queries = nullptr;
     } order;
     unsigned int* d_trace = nullptr;
     uint32_t trace_ns = 0;

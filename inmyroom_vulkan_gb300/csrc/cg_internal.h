@@ -251,12 +251,12 @@ struct LeafOrderParams {
     const uint4* leaf_list;
     const unsigned long long* n_leafs;
     uint32_t leaf_cap;
-    const ulonglong2* keys;   // launch_leaf_keys' results
+    const ulonglong2* keys;   // launch_leaf_keys' results (key[1] and index[1] may be keys and place)
     const uint32_t* count;
     const uint32_t* place;
     uint32_t* first;          // [n_queries] scratch: each query's first place
     uint32_t* tile;           // [n_queries + 1] scratch: its first tile
-    ulonglong2* key[2];       // [leaf_cap] scratch
+    ulonglong2* key[2];       // [leaf_cap] scratch (key[0] may be out)
     uint32_t* index[2];
     cg_leaf_pair* out;
 };

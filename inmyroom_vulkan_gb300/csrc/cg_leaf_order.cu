@@ -16,6 +16,14 @@
 //                 written out. As many launches as the largest possible list
 //                 needs (a list that needs fewer ends them at once)
 //
+// Of the two buffers of paths the first is the output's own memory (a record
+// has a path's size) and the second the list-ordered paths', done with once
+// they are grouped; the second buffer of indexes is the places'. So a leaf pair
+// takes 24 bytes beside the list and the output (60 with buffers of their own).
+// A tile is read before its block writes it out; a merge that reads the first
+// buffer leaves the query for the next one, which reads the second, to write
+// out.
+//
 // All of it is memory latency: 155,000 leaf pairs of 250 queries take 67 us
 // (tiles 32, merges 26) where reading paths and pairs back and sorting them on
 // the host took 3.6 ms.
@@ -33,6 +41,7 @@ __device__ __forceinline__ uint32_t listed(const LeafOrderParams& P) {
     const unsigned long long n = *reinterpret_cast<const volatile unsigned long long*>(P.n_leafs);
     return uint32_t(n < P.leaf_cap ? n : P.leaf_cap);
 }
+static_assert(sizeof(cg_leaf_pair) == sizeof(ulonglong2), "the output's memory holds a path per leaf pair");
 __device__ __forceinline__ bool before(ulonglong2 a, ulonglong2 b) { return a.x < b.x || (a.x == b.x && a.y < b.y); }
 
 // Leaf pair i of the list, as read back, to place pos.
@@ -136,8 +145,8 @@ __global__ void __launch_bounds__(512) leaf_tiles_kernel(const LeafOrderParams P
             if (count <= kLeafTile) {
                 emit(P, base + k, id[k]);
             } else {
-                P.key[0][base + k] = key[k];
-                P.index[0][base + k] = id[k];
+                P.key[1][base + k] = key[k];
+                P.index[1][base + k] = id[k];
             }
         }
         __syncthreads();
@@ -159,7 +168,10 @@ __global__ void __launch_bounds__(256) leaf_merge_kernel(const LeafOrderParams P
                 b = m - 1u;
         }
         const uint32_t first = P.first[a], count = P.count[a];
-        if (count <= run) continue;  // written out already
+        if (count <= run) {  // written out already, or one run since the merge before this one
+            if (from == 1u && run > kLeafTile && count > run / kLeafWays) emit(P, pos, P.index[1][pos]);
+            continue;
+        }
         const uint32_t i = P.index[from][pos];
         const ulonglong2 k = key[pos];
         const uint64_t wide = run * kLeafWays, local = pos - first, group = local / wide * wide;
@@ -181,7 +193,7 @@ __global__ void __launch_bounds__(256) leaf_merge_kernel(const LeafOrderParams P
             rank += lo;
         }
         const uint32_t to = uint32_t(first + group + rank);
-        if (count <= wide) {
+        if (from == 1u && count <= wide) {
             emit(P, to, i);
         } else {
             P.key[from ^ 1u][to] = k;
@@ -196,8 +208,9 @@ cudaError_t launch_leaf_order(const LeafOrderParams& p, uint32_t sm_count, cudaS
     leaf_offsets_kernel<<<1, 1024, 0, s>>>(p);
     leaf_group_kernel<<<8u * sm_count, 256, 0, s>>>(p);
     leaf_tiles_kernel<<<4u * sm_count, 512, 0, s>>>(p);
-    uint32_t from = 0;
-    for (uint64_t run = kLeafTile; run < p.leaf_cap; run *= kLeafWays, from ^= 1u)
+    uint32_t from = 1;
+    // (the last merge is one that writes out)
+    for (uint64_t run = kLeafTile; run < p.leaf_cap || (from == 1u && run > kLeafTile); run *= kLeafWays, from ^= 1u)
         leaf_merge_kernel<<<8u * sm_count, 256, 0, s>>>(p, run, from);
     return cudaGetLastError();
 }
