@@ -531,14 +531,13 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
                                 c->ev_branch, c->ev_branched), "contact kernels");
     }
     if (pairs_copy) CG_CUDA(cudaStreamWaitEvent(s, c->ev_joined, 0), "join");
-    // a captured step (here or by the caller) may be replayed without a call:
-    // it leaves its counters on the host itself
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    CG_CUDA(cudaStreamIsCapturing(s, &st), "capture status");
-    if (st == cudaStreamCaptureStatusNone)
-        c->ctr_mirrored = false;
-    else
+    // a captured step is replayed without this call: it leaves its counters on
+    // the host itself (the caller's own capture cannot take a step, whose
+    // results the context's stream waits for)
+    if (c->capturing)
         CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s), "copy counters");
+    else
+        c->ctr_mirrored = false;
     return CG_OK;
 }
 
