@@ -212,12 +212,13 @@ __device__ int poll_ready(const TraverseParams& P, uint32_t slot, unsigned long 
     return -1;
 }
 
+// Adds v busy lanes in `steps` warps' steps to the bucket of the present time.
 __device__ __forceinline__ void trace_add(unsigned int* trace, uint32_t trace_ns, unsigned long long t_base, int field,
-                                          unsigned v) {
+                                          unsigned v, unsigned steps) {
     const unsigned long long b = (gtimer() - t_base) / trace_ns;
     if (b < kTraceBuckets) {
         atomicAdd(trace + 4 * b + field, v);
-        atomicAdd(trace + 4 * b + field + 1, 1u);
+        atomicAdd(trace + 4 * b + field + 1, steps);
     }
 }
 
@@ -393,7 +394,7 @@ __device__ __forceinline__ void narrow_block(const NarrowParams& P, uint32_t* st
         const unsigned kept = __ballot_sync(kFull, keep);
         if (keep) Q.e[Q.n + __popc(kept & lanemask_lt())] = e;
         Q.n += __popc(kept);
-        if (lane == 0 && P.trace) trace_add(P.trace, P.trace_ns, t_base, 2, min(32u, total - base));
+        if (lane == 0 && P.trace) trace_add(P.trace, P.trace_ns, t_base, 2, min(32u, total - base), 1u);
         if (Q.n >= 32u) narrow_run<kMode>(P, Q, 32u, lane, N);
     }
     if (lane == 0) N.tests += total;
@@ -650,8 +651,9 @@ __global__ void __launch_bounds__(kWorkerMax * 32, 2) traverse_kernel(const Trav
         if (tid == 0) {
             sh.qs[par] = qs;
             st_nodes += 2u * n;
-            st_steps += ((n << lg) + 31u) >> 5;  // steps of warps that hold items
-            if (P.trace) trace_add(P.trace, P.trace_ns, t_base, 0, n);
+            const uint32_t steps = ((n << lg) + 31u) >> 5;  // of warps that hold items
+            st_steps += steps;
+            if (P.trace) trace_add(P.trace, P.trace_ns, t_base, 0, n, steps);
         }
         __syncthreads();
         const unsigned pushed = sh.push[par];
