@@ -2,7 +2,7 @@
 // the persistent warp-cooperative OBB-tree traversal, and the persistent
 // triangle-pair (Moller) narrow phase.
 //
-// Traversal. A worker is a block of two or four warps that share a deque of
+// Traversal. A worker is a block of one, two or four warps that share a deque of
 // items in shared memory and advance it a step at a time: up to 32 items per
 // warp, an item being a split node whose two children are tested against the
 // other tree's box. A step loads the box records (four 16-byte loads each) and
@@ -884,7 +884,11 @@ namespace {
 // Traversal alone, 1, 2, 4 and 8 warps (us): 1 query of 2 x 2,048 triangles
 // 59, 51, 48, 47; 64 of these 85, 67, 58, 64; 150 queries of 2 x 20,000 213,
 // 180, 190, 202; the 256-entity scene 131, 103, 110, 119; 10,000 uneven
-// queries 1310, 1288, 1392, 1587.
+// queries 1310, 1288, 1392, 1587. The line is where a worker of four warps still
+// has a query of its own to itself; from 64 queries up to it two warps are
+// somewhat faster for large trees (150 queries: 180 against 190), four for small
+// ones.
+//
 // With the smallest stacks (256 entries) a worker is one warp and takes one root
 // at a time: donations that a full stack forces are then the rule, and how many
 // of the queue's slots they take decides whether a launch fits its queue. Two
