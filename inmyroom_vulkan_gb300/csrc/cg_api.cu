@@ -54,9 +54,9 @@ void free_buffers(cg_ctx* c) {
     cudaFree(c->d_ready);
     cudaFree(c->d_pairs);
     cudaFree(c->d_leafs);
-    for (void* p : {(void*)c->order.keys, (void*)c->order.place, (void*)c->order.index, (void*)c->order.queries})
-        cudaFree(p);
+    cudaFree(c->order.keys);
     c->order = cg_ctx::LeafOrder{};
+    c->order_queries = 0;
     cudaFree(c->d_trace);
     auto& t = c->ct;
     for (void* p : {(void*)t.pair_aux, (void*)t.table, (void*)t.occupied, (void*)t.slot_info, (void*)t.big_slots, (void*)t.pg_geom, (void*)t.pg_link,
@@ -379,12 +379,19 @@ void put_box(float4* rec, const cg_obb& b, uint32_t ref, uint32_t meta, uint32_t
     rec[3] = make_float4(r, m, 0.f, sp);
 }
 
+// What the reads after a step need to know of it, once it is enqueued.
+void step_started(cg_ctx* c, uint32_t n, uint32_t flags, bool mirrored) {
+    c->ctr_mirrored = mirrored;
+    c->order_queries = (flags & CG_DFS_ORDER) ? n : 0u;
+}
+
 // Enqueues counter reset, packing, the traversal and the narrow phase on `s`.
 // pairs_copy: with the step's colliding pairs final (after the narrow phase),
 // copy them out on a branch that runs beside the contact kernels.
 int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flags, cudaStream_t s,
                  const CopyOutParams* pairs_copy, const CopyOutParams* results_copy) {
     c->last_n = n;
+    if (!c->capturing) step_started(c, 0, 0, false);
     unsigned int* trace = (flags & CG_TRACE) ? c->d_trace : nullptr;
     const uint32_t trace_ns = c->trace_ns ? c->trace_ns : 1000u;
     CG_CUDA(launch_init(c->d_ctr, c->d_ready, c->slot_alloc, n, trace, s), "init kernel");
@@ -420,7 +427,7 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
     np.pairs_cap = c->d_pairs ? c->cfg.max_tri_pairs : 0;
     np.leafs = c->d_leafs;
     np.leafs_cap = c->d_leafs ? c->cfg.max_leaf_pairs : 0;
-    // ordered leaf pairs are written by the ordering kernels
+    // ordered leaf pairs are written when they are read
     np.flags = (flags & CG_DFS_ORDER) ? flags & ~CG_KEEP_LEAF_PAIRS : flags;
     np.trace = trace;
     np.trace_ns = trace_ns;
@@ -442,25 +449,9 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
         kp.keys = c->order.keys;
         kp.count = c->order.queries;
         kp.place = c->order.place;
+        kp.most = &c->d_ctr->order_most;
         CG_CUDA(cudaMemsetAsync(kp.count, 0, sizeof(uint32_t) * n, s), "clear leaf-pair counts");
         CG_CUDA(launch_leaf_keys(kp, c->contact_blocks, s), "leaf-pair key kernel");
-        LeafOrderParams op{};
-        op.q = c->d_packed;
-        op.n_queries = n;
-        op.leaf_list = c->d_leaf_list;
-        op.n_leafs = kp.n_leafs;
-        op.leaf_cap = p.leaf_cap;
-        op.keys = kp.keys;
-        op.count = kp.count;
-        op.place = kp.place;
-        op.first = kp.count + c->cfg.max_queries;
-        op.tile = op.first + c->cfg.max_queries;
-        op.out = c->d_leafs;
-        op.key[0] = reinterpret_cast<ulonglong2*>(c->d_leafs);
-        op.key[1] = c->order.keys;
-        op.index[0] = c->order.index;
-        op.index[1] = c->order.place;
-        CG_CUDA(launch_leaf_order(op, uint32_t(c->sm_count), s), "leaf-pair order kernels");
     }
     if (pairs_copy) {
         CG_CUDA(cudaEventRecord(c->ev_fork, s), "fork event");
@@ -537,7 +528,7 @@ int enqueue_step(cg_ctx* c, const cg_query* d_queries, uint32_t n, uint32_t flag
     if (c->capturing)
         CG_CUDA(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s), "copy counters");
     else
-        c->ctr_mirrored = false;
+        step_started(c, n, flags, false);
     return CG_OK;
 }
 
@@ -606,12 +597,13 @@ int check_flags(cg_ctx* c, uint32_t flags) {
             return fail(c, CG_ERR_INVALID_ARGUMENT, "CG_DFS_ORDER orders the kept leaf pairs: it needs "
                         "CG_KEEP_LEAF_PAIRS and max_leaf_pairs > 0");
         auto& o = c->order;
-        const uint64_t m = c->cfg.max_leaf_pairs;
-        if (!o.queries) {
-            if (!o.keys) CG_CUDA(cudaMalloc(&o.keys, sizeof(ulonglong2) * m), "alloc leaf-pair keys");
-            if (!o.place) CG_CUDA(cudaMalloc(&o.place, sizeof(uint32_t) * m), "alloc leaf-pair places");
-            if (!o.index) CG_CUDA(cudaMalloc(&o.index, sizeof(uint32_t) * m), "alloc leaf-pair order");
-            CG_CUDA(cudaMalloc(&o.queries, sizeof(uint32_t) * (3ull * c->cfg.max_queries + 1u)), "alloc leaf-pair order");
+        const uint64_t m = c->cfg.max_leaf_pairs, mq = c->cfg.max_queries;
+        if (!o.keys) {
+            CG_CUDA(cudaMalloc(&o.keys, sizeof(ulonglong2) * m + sizeof(uint32_t) * (2u * m + 3u * mq + 1u)),
+                    "alloc leaf-pair order");
+            o.place = reinterpret_cast<uint32_t*>(o.keys + m);
+            o.index = o.place + m;
+            o.queries = o.index + m;
         }
     }
     if (!(flags & CG_CONTACTS)) return CG_OK;
@@ -1107,7 +1099,7 @@ int cg_collide(cg_ctx* c, const cg_query* queries, uint32_t n, uint32_t flags, c
         G.out_gen = c->host_out.gen;
     }
     CG_CUDA(cudaGraphLaunch(G.exec, c->stream), "collide step");
-    c->ctr_mirrored = true;
+    step_started(c, n, flags, true);
     CG_CUDA(cudaStreamSynchronize(c->stream), "collide");
     return stats_from(c, *c->h_ctr, st);
 }
@@ -1166,8 +1158,30 @@ int cg_read_leaf_pairs(cg_ctx* c, cg_leaf_pair* out, uint64_t cap, uint64_t* n) 
     const uint64_t avail = std::min<uint64_t>(c->h_ctr->n_leafs, c->d_leafs ? c->cfg.max_leaf_pairs : 0);
     *n = c->h_ctr->n_leafs;
     const uint64_t m = std::min(avail, cap);
+    if (m && c->order_queries) {
+        LeafOrderParams op{};
+        op.q = c->d_packed;
+        op.n_queries = c->order_queries;
+        op.leaf_list = c->d_leaf_list;
+        op.n = uint32_t(avail);
+        op.most = c->h_ctr->order_most;
+        op.keys = c->order.keys;
+        op.count = c->order.queries;
+        op.place = c->order.place;
+        op.first = c->order.queries + c->cfg.max_queries;
+        op.tile = op.first + c->cfg.max_queries;
+        op.out = c->d_leafs;
+        op.key[0] = reinterpret_cast<ulonglong2*>(c->d_leafs);
+        op.key[1] = c->order.keys;
+        op.index[0] = c->order.index;
+        op.index[1] = c->order.place;
+        CG_CUDA(launch_leaf_order(op, uint32_t(c->sm_count), c->stream), "leaf-pair order kernels");
+        c->order_queries = 0;
+    }
     if (m) {
-        CG_CUDA(cudaMemcpy(out, c->d_leafs, sizeof(cg_leaf_pair) * m, cudaMemcpyDeviceToHost), "read leaf pairs");
+        CG_CUDA(cudaMemcpyAsync(out, c->d_leafs, sizeof(cg_leaf_pair) * m, cudaMemcpyDeviceToHost, c->stream),
+                "read leaf pairs");
+        CG_CUDA(cudaStreamSynchronize(c->stream), "read leaf pairs");
     }
     return c->h_ctr->n_leafs > avail ? CG_ERR_OUTPUT_OVERFLOW : CG_OK;
 }
@@ -1541,7 +1555,7 @@ int cg_graph_launch(cg_ctx* c, void* stream) {
     cudaSetDevice(c->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->stream;
     CG_CUDA(cudaGraphLaunch(c->graph_exec, s), "graph launch");
-    c->ctr_mirrored = true;
+    step_started(c, c->graph_n, c->graph_flags, true);
     c->last_flags = c->graph_flags;
     c->last_n = c->graph_n;
     return join_stream(c, s);

@@ -1852,12 +1852,16 @@ __global__ void __launch_bounds__(kPathWarps * 32) leaf_keys_kernel(const LeafKe
         unsigned long long hi, lo;
         uint32_t depth;
         paired_path(P.q, P.trees, P.recs, lp, valid, way[wib], hi, lo, depth);
+        uint32_t count = 0;
         if (!(lane & 1u) && valid) {
             if (depth >= 128u) atomicOr(P.error, ERR_DEEP);
             P.keys[i] = make_ulonglong2(hi, lo);
-            P.place[i] = atomicAdd(P.count + lp.x, 1u);
+            const uint32_t place = atomicAdd(P.count + lp.x, 1u);
+            P.place[i] = place;
+            count = place + 1u;
         }
-        __syncwarp();
+        count = __reduce_max_sync(0xffffffffu, count);
+        if (lane == 0u) atomicMax(P.most, count);
     }
 }
 

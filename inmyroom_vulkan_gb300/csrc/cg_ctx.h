@@ -139,9 +139,9 @@ struct cg_ctx {
     uint4* d_leaf_list = nullptr;   // candidate leaf pairs between the two kernels
     cg_tri_pair* d_pairs = nullptr;
     cg_leaf_pair* d_leafs = nullptr;
-    // CG_DFS_ORDER, allocated on first use: each leaf pair's descent path and
-    // number within its query (the sort's second buffers, too), the sort's
-    // indexes, the queries' counts and places
+    // CG_DFS_ORDER, one block allocated on first use: each leaf pair's descent
+    // path and number within its query (the sort's second buffers, too), the
+    // sort's indexes, the queries' counts and places
     struct LeafOrder {
         ulonglong2* keys = nullptr;
         uint32_t *place = nullptr, *index = nullptr, *queries = nullptr;
@@ -189,6 +189,7 @@ struct cg_ctx {
     cg_query* h_queries = nullptr;  // pinned
     Counters* h_ctr = nullptr;      // pinned
     bool ctr_mirrored = false;      // h_ctr holds the last launch's counters once the stream's work is done
+    uint32_t order_queries = 0;     // queries of a CG_DFS_ORDER launch whose leaf pairs are still to be ordered (0: none)
 
     uint32_t last_flags = 0;
     uint32_t last_n = 0;            // queries of the last collide step enqueued

@@ -100,6 +100,7 @@ struct Counters {
     unsigned int order_big_ticket;  // larger maps taken
     unsigned int n_bigmaps;      // larger maps
     unsigned int n_wholemaps;    // maps of kHalfMap triangles or more
+    unsigned int order_most;     // leaf pairs of the query with the most (CG_DFS_ORDER)
     unsigned int n_big;          // contact slots of more than kFoldThread contributions (listed for the fold)
     unsigned int fold_done;      // fold blocks finished (the last one ranks the maps)
     unsigned int order_done;     // order blocks finished (the last one places the maps' records and rays)
@@ -241,6 +242,7 @@ struct LeafKeyParams {
     ulonglong2* keys;                   // per leaf pair: path high, low
     uint32_t* count;                    // per query: its leaf pairs (zero before the launch)
     uint32_t* place;                    // per leaf pair: its number within its query
+    uint32_t* most;                     // the largest count (zero before the launch)
 };
 cudaError_t launch_leaf_keys(const LeafKeyParams& p, uint32_t grid, cudaStream_t s);
 
@@ -249,14 +251,13 @@ struct LeafOrderParams {
     const PackedQuery* q;
     uint32_t n_queries;
     const uint4* leaf_list;
-    const unsigned long long* n_leafs;
-    uint32_t leaf_cap;
+    uint32_t n, most;         // leaf pairs in the list, and of the query with the most
     const ulonglong2* keys;   // launch_leaf_keys' results (key[1] and index[1] may be keys and place)
     const uint32_t* count;
     const uint32_t* place;
     uint32_t* first;          // [n_queries] scratch: each query's first place
     uint32_t* tile;           // [n_queries + 1] scratch: its first tile
-    ulonglong2* key[2];       // [leaf_cap] scratch (key[0] may be out)
+    ulonglong2* key[2];       // [n] scratch (key[0] may be out)
     uint32_t* index[2];
     cg_leaf_pair* out;
 };

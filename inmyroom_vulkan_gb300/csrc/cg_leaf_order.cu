@@ -1,7 +1,16 @@
 // The candidate leaf pairs of a CG_DFS_ORDER step in the order of the
 // reference's recursion (OBBtree::IntersectOBBtreesRecursive,
 // src/Geometry/OBBtree.cpp:414-476): grouped by query, each query's by the
-// 128-bit descent paths that leaf_keys_kernel (cg_contacts.cu) found.
+// 128-bit descent paths that leaf_keys_kernel (cg_contacts.cu) found. Ordered
+// when they are first read: their numbers are known by then, so that only the
+// launches that the list needs are made, none for an empty one (in the step,
+// with launches for the longest possible list, one pair's mid phase without
+// leaf pairs took 76 us instead of 60).
+//
+//   leaf_few      a list of at most a tile: one block sorts it by query and path
+//                 and writes it out
+//
+// A longer one:
 //
 //   leaf_offsets  one block: the queries' places (prefix sums of their counts,
 //                 which leaf_keys counted) and their tiles of kLeafTile
@@ -13,8 +22,8 @@
 //                 32 sorted runs is its place in its own plus its lower bounds
 //                 in the others (independent binary searches), so each launch
 //                 makes runs 32 times longer; a query that is one run is
-//                 written out. As many launches as the largest possible list
-//                 needs (a list that needs fewer ends them at once)
+//                 written out. As many launches as the query with the most
+//                 needs
 //
 // Of the two buffers of paths the first is the output's own memory (a record
 // has a path's size) and the second the list-ordered paths', done with once
@@ -37,10 +46,6 @@ namespace {
 
 constexpr uint32_t kLeafTile = 1024, kLeafWays = 32;
 
-__device__ __forceinline__ uint32_t listed(const LeafOrderParams& P) {
-    const unsigned long long n = *reinterpret_cast<const volatile unsigned long long*>(P.n_leafs);
-    return uint32_t(n < P.leaf_cap ? n : P.leaf_cap);
-}
 static_assert(sizeof(cg_leaf_pair) == sizeof(ulonglong2), "the output's memory holds a path per leaf pair");
 __device__ __forceinline__ bool before(ulonglong2 a, ulonglong2 b) { return a.x < b.x || (a.x == b.x && a.y < b.y); }
 
@@ -55,6 +60,37 @@ __device__ __forceinline__ void emit(const LeafOrderParams& P, uint32_t pos, uin
     lp.count_a = uint16_t(e.w & 0xffffu);
     lp.count_b = uint16_t(e.w >> 16);
     P.out[pos] = lp;
+}
+
+// Entry of leaf_few's sort.
+struct FewKey {
+    ulonglong2 path;
+    uint32_t query, id;
+};
+__device__ __forceinline__ bool before(const FewKey& a, const FewKey& b) {
+    if (a.query != b.query) return a.query < b.query;
+    if (a.path.x != b.path.x) return a.path.x < b.path.x;
+    return a.path.y != b.path.y ? a.path.y < b.path.y : a.id < b.id;
+}
+
+__global__ void __launch_bounds__(512) leaf_few_kernel(const LeafOrderParams P) {
+    __shared__ FewKey key[kLeafTile];
+    const uint32_t tid = threadIdx.x;
+    uint32_t size = 1;
+    while (size < P.n) size <<= 1;
+    for (uint32_t k = tid; k < size; k += 512u)
+        key[k] = k < P.n ? FewKey{P.keys[k], P.leaf_list[k].x, k} : FewKey{make_ulonglong2(~0ull, ~0ull), ~0u, ~0u};
+    __syncthreads();
+    for (uint32_t width = 2; width <= size; width <<= 1)
+        for (uint32_t step = width >> 1; step; step >>= 1) {
+            for (uint32_t p = tid; p < size / 2u; p += 512u) {
+                const uint32_t i = 2u * p - (p & (step - 1u)), j = i + step;
+                const FewKey x = key[i], y = key[j];
+                if (before(y, x) == ((i & width) == 0u)) key[i] = y, key[j] = x;
+            }
+            __syncthreads();
+        }
+    for (uint32_t k = tid; k < P.n; k += 512u) emit(P, k, key[k].id);
 }
 
 __global__ void __launch_bounds__(1024) leaf_offsets_kernel(const LeafOrderParams P) {
@@ -95,8 +131,7 @@ __global__ void __launch_bounds__(1024) leaf_offsets_kernel(const LeafOrderParam
 }
 
 __global__ void __launch_bounds__(256) leaf_group_kernel(const LeafOrderParams P) {
-    const uint32_t n = listed(P);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += gridDim.x * blockDim.x) {
         const uint32_t pos = P.first[P.leaf_list[i].x] + P.place[i];
         P.key[0][pos] = P.keys[i];
         P.index[0][pos] = i;
@@ -155,9 +190,8 @@ __global__ void __launch_bounds__(512) leaf_tiles_kernel(const LeafOrderParams P
 
 // Merges runs of `run` leaf pairs, from buffer `from` into the other.
 __global__ void __launch_bounds__(256) leaf_merge_kernel(const LeafOrderParams P, uint64_t run, uint32_t from) {
-    const uint32_t n = listed(P);
     const ulonglong2* key = P.key[from];
-    for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += gridDim.x * blockDim.x) {
+    for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < P.n; pos += gridDim.x * blockDim.x) {
         // its query: the last whose first place is at or before pos
         uint32_t a = 0, b = P.n_queries - 1u;
         while (a < b) {
@@ -205,12 +239,17 @@ __global__ void __launch_bounds__(256) leaf_merge_kernel(const LeafOrderParams P
 }  // namespace
 
 cudaError_t launch_leaf_order(const LeafOrderParams& p, uint32_t sm_count, cudaStream_t s) {
+    if (p.n == 0) return cudaSuccess;
+    if (p.n <= kLeafTile) {
+        leaf_few_kernel<<<1, 512, 0, s>>>(p);
+        return cudaGetLastError();
+    }
     leaf_offsets_kernel<<<1, 1024, 0, s>>>(p);
     leaf_group_kernel<<<8u * sm_count, 256, 0, s>>>(p);
     leaf_tiles_kernel<<<4u * sm_count, 512, 0, s>>>(p);
     uint32_t from = 1;
     // (the last merge is one that writes out)
-    for (uint64_t run = kLeafTile; run < p.leaf_cap || (from == 1u && run > kLeafTile); run *= kLeafWays, from ^= 1u)
+    for (uint64_t run = kLeafTile; run < p.most || (from == 1u && run > kLeafTile); run *= kLeafWays, from ^= 1u)
         leaf_merge_kernel<<<8u * sm_count, 256, 0, s>>>(p, run, from);
     return cudaGetLastError();
 }

@@ -35,7 +35,7 @@ def test_more_than_two_merges(port):
         assert np.array_equal(rows(ctx.leaf_pairs()), want)
 
 
-@pytest.mark.parametrize("cap", [1, 700, 5000, 60000])
+@pytest.mark.parametrize("cap", [1, 2, 31, 700, 1023, 1024, 1025, 5000, 60000])
 def test_overflowed_list_is_grouped_and_ordered(port, cap):
     trees, want = spheres(port, 5, 0.01)
     place = {tuple(r): i for i, r in enumerate(want.tolist())}
@@ -64,3 +64,28 @@ def test_memory_of_the_first_ordered_step(port):
         free = torch.cuda.mem_get_info()[0]
         ctx.collide(q, FLAGS)
         assert free - torch.cuda.mem_get_info()[0] <= 24 * cap + (16 << 20)
+
+
+def test_order_belongs_to_the_step_that_ran(port):
+    """A capture between a step and its reads changes neither's leaf pairs, and a second read returns the first's."""
+    torch = pytest.importorskip("torch")
+    trees, want = spheres(port, 4, 0.01)
+    with capi.Context() as ctx:
+        a, b = (ctx.upload_flat(t.export()) for t in trees)
+        q = capi.make_queries([a, b, a], [b, a, b], np.stack([capi.relative_matrix(EYE, EYE)] * 3))
+        d_q = torch.from_numpy(q.view(np.uint8).copy()).cuda()
+        torch.cuda.synchronize()
+        plain = capi.CG_KEEP_LEAF_PAIRS | capi.CG_MID_ONLY
+        ctx.collide(q[:1], FLAGS)
+        ctx.graph_capture(d_q.data_ptr(), 3, plain)
+        for _ in range(2):
+            assert np.array_equal(rows(ctx.leaf_pairs()), want)
+        ctx.graph_launch()  # unordered, of three queries
+        lp = ctx.leaf_pairs()
+        assert len(lp) > 2 * len(want) and sorted(map(tuple, rows(lp[lp["query"] == 2]).tolist())) == sorted(map(tuple, want.tolist()))
+        ctx.graph_capture(d_q.data_ptr(), 1, FLAGS)
+        again = ctx.leaf_pairs()
+        assert np.array_equal(again, lp)
+        for _ in range(2):
+            ctx.graph_launch()
+            assert np.array_equal(rows(ctx.leaf_pairs()), want)
